@@ -1,0 +1,288 @@
+// Attention on warp-level MMAs for 16-bit tensors that the tcgen05 kernels do not take (head_dim other than 128, or views
+// that a TMA map cannot describe), with the accuracy of f32 arithmetic.
+//
+// The products q.k of 16-bit values are exact in f32, so S = Q K^T loses nothing on the tensor cores.  The softmax weights do
+// not fit 16 bits: they are handed over as a sum of 16-bit terms, two for f16 (22 significant bits) and three for bf16 (24),
+// each multiplied by the same V fragment.  The tcgen05 kernels keep one 11-bit term; callers of this path had f32 arithmetic
+// before (general_attention_kernel) and keep it.
+//
+// One CTA = 64 query rows of one (batch, head), 4 warps x 16 rows; K and V tiles of 64 keys come by cp.async into two
+// buffers, rows padded by 16 bytes so that ldmatrix meets no bank conflict; Q stays in registers.  Three CTAs per SM
+// (head_dim 64) hide each other's barriers and softmax.  Bound by the warp MMA pipe (538 TFLOP/s of bf16 products, measured):
+// B4 H32/8 S2048 D64 causal 201 TFLOP/s in f16 and 158 in bf16, three and four MMAs per useful two, 55-59 % of that pipe.
+// Against the f32-arithmetic kernel that served these tensors: B8 H16 S300 D64 f16 with a key mask 852 -> 31 us, B2 H32/8 S1024
+// D64 bf16 causal 2259 -> 64 us; error against 64 bits 2.1e-7 to 3.7e-7 of the norm (f32 arithmetic: 1.7e-7 to 8.7e-7).
+#pragma once
+#include "ptx_sm100.cuh"
+
+namespace fusor {
+
+constexpr int AM_BM = 64, AM_BN = 64, AM_THREADS = 128;
+
+struct AttnMmaParams {
+    const void* q;
+    const void* k;
+    const void* v;
+    void* out;
+    const float* mask;
+    int out_dtype;  // 0 = f32, 1 = bf16, 2 = f16
+    int B, Hq, Hkv, Sq, Skv, D;
+    long long qs[3], ks[3], vs[3], os[3];  // element strides of batch, head, row
+    long long ms[2];                       // mask strides
+    int mask_kind;                         // FUSOR_CUDA_MASK_*
+    int window;
+    int n_q_tiles;
+    float scale;
+};
+
+__device__ __forceinline__ void cp_async16_zfill(uint32_t smem, const void* gmem, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem), "l"(gmem), "r"(valid ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// c (16x8, f32) += a (16x16, row) * b (16x8, col), both f16 or both bf16
+template <bool F16>
+__device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    if (F16)
+        asm volatile(
+            "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+            : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+            : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+    else
+        mma_bf16_16816(c, a, b0, b1);
+}
+
+// Two f32 -> packed 16-bit pair; x and y keep what the pair does not hold.
+template <bool F16>
+__device__ __forceinline__ uint32_t split_pair(float& x, float& y) {
+    if (F16) {
+        const __half2 h = __floats2half2_rn(x, y);
+        const float2 f = __half22float2(h);
+        x -= f.x;
+        y -= f.y;
+        return *reinterpret_cast<const uint32_t*>(&h);
+    }
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+    x -= __low2float(h);
+    y -= __high2float(h);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+template <int DP>
+constexpr int am_pitch = DP * 2 + 16;  // bytes of a row in shared memory
+template <int DP>
+constexpr size_t am_smem_bytes = (size_t)am_pitch<DP> * (AM_BM + 4 * AM_BN);
+
+// Online softmax of row r (0 or 1) of the thread's fragment: a row lives in the four threads of a quad.  m is the row maximum
+// in log2 units, l this thread's part of the row sum.  s becomes the weights.
+template <int BN, bool ADD>
+__device__ __forceinline__ void am_softmax_row(float (&s)[BN / 8][4], int r, float c, float2 c2, float& m, float& l, float& alpha) {
+    float mx = fmaxf(s[0][2 * r], s[0][2 * r + 1]);
+#pragma unroll
+    for (int nt = 1; nt < BN / 8; ++nt) mx = fmax3(mx, s[nt][2 * r], s[nt][2 * r + 1]);
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+    mx = fmaxf(m, ADD ? mx : mx * c);
+    // a row whose keys so far are all masked keeps m = -inf: subtract 0, so that its weights are 0 and not NaN
+    const float ms = mx == -INFINITY ? 0.0f : mx;
+    const float2 nm2 = make_float2(-ms, -ms);
+    alpha = fast_exp2(m - ms);
+    m = mx;
+    float2 sum = make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int nt = 0; nt < BN / 8; ++nt) {
+        const float2 x = ffma2(make_float2(s[nt][2 * r], s[nt][2 * r + 1]), c2, nm2);
+        const float2 p = make_float2(fast_exp2(x.x), fast_exp2(x.y));
+        s[nt][2 * r] = p.x;
+        s[nt][2 * r + 1] = p.y;
+        sum = fadd2(sum, p);
+    }
+    l = l * alpha + (sum.x + sum.y);
+}
+
+// o = o alpha + t
+template <int DP>
+__device__ __forceinline__ void am_accumulate(float (&o)[DP / 8][4], const float (&t)[DP / 8][4], const float (&alpha)[2]) {
+#pragma unroll
+    for (int nd = 0; nd < DP / 8; ++nd)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const float2 x = ffma2(make_float2(o[nd][2 * r], o[nd][2 * r + 1]), make_float2(alpha[r], alpha[r]), make_float2(t[nd][2 * r], t[nd][2 * r + 1]));
+            o[nd][2 * r] = x.x;
+            o[nd][2 * r + 1] = x.y;
+        }
+}
+
+// O / l (a fully masked row gives 0 * inf = NaN, as the reference)
+template <int DP>
+__device__ __forceinline__ void am_store(const AttnMmaParams& P, const float (&o)[DP / 8][4], float (&l)[2], int r0, int cq, int b, int h) {
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        l[r] += __shfl_xor_sync(0xffffffffu, l[r], 1);
+        l[r] += __shfl_xor_sync(0xffffffffu, l[r], 2);
+        const int qi = r0 + r * 8;
+        if (qi >= P.Sq) continue;
+        const float inv = 1.0f / l[r];
+        const long long row = b * P.os[0] + h * P.os[1] + qi * P.os[2];
+#pragma unroll
+        for (int nd = 0; nd < DP / 8; ++nd) {
+            const int d = nd * 8 + cq;
+            if (d >= P.D) continue;
+            if (P.out_dtype == 0) *reinterpret_cast<float2*>(static_cast<float*>(P.out) + row + d) = make_float2(o[nd][2 * r] * inv, o[nd][2 * r + 1] * inv);
+            else *reinterpret_cast<uint32_t*>(static_cast<uint16_t*>(P.out) + row + d) = pack_16(P.out_dtype, o[nd][2 * r] * inv, o[nd][2 * r + 1] * inv);
+        }
+    }
+}
+
+// DP: head_dim rounded up to 32; columns D.. of Q, K and V read as zero
+// ADD: an additive mask tensor is read
+template <int DP, bool F16, bool ADD>
+__global__ void __launch_bounds__(AM_THREADS, DP <= 64 ? 3 : 2) attn_mma16_kernel(const __grid_constant__ AttnMmaParams P) {
+    extern __shared__ __align__(16) uint8_t am_smem[];
+    constexpr int PITCH = am_pitch<DP>, CH = DP / 8;  // 16-byte chunks of a row
+    constexpr int TERMS = F16 ? 2 : 3;
+    constexpr float LOG2E = 1.4426950408889634f;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t q_sm = smem_u32(am_smem);
+    const uint32_t kv_sm = q_sm + AM_BM * PITCH;  // [2 buffers]{K, V}
+
+    // heavy (late) row blocks first
+    const int qt = P.n_q_tiles - 1 - (int)(blockIdx.x / (unsigned)(P.Hq * P.B));
+    const int hb = (int)(blockIdx.x % (unsigned)(P.Hq * P.B));
+    const int h = hb % P.Hq, b = hb / P.Hq, hk = h / (P.Hq / P.Hkv);
+    const int q0 = qt * AM_BM;
+    const int offset = P.Skv - P.Sq;  // causal: key k allowed iff k <= q + offset
+    const bool causal = P.mask_kind == 3 || P.mask_kind == 4;
+    int k_begin = 0, k_end = P.Skv;
+    if (causal) {
+        k_end = min(P.Skv, min(q0 + AM_BM, P.Sq) + offset);
+        if (P.mask_kind == 4) k_begin = max(0, q0 + offset - P.window + 1) / AM_BN * AM_BN;
+    }
+    const uint16_t* qg = static_cast<const uint16_t*>(P.q) + b * P.qs[0] + h * P.qs[1];
+    const uint16_t* kg = static_cast<const uint16_t*>(P.k) + b * P.ks[0] + hk * P.ks[1];
+    const uint16_t* vg = static_cast<const uint16_t*>(P.v) + b * P.vs[0] + hk * P.vs[1];
+
+    auto load_rows = [&](uint32_t dst, const uint16_t* src, long long row_stride, int row0, int rows_end) {
+#pragma unroll
+        for (int i = tid; i < 64 * CH; i += AM_THREADS) {
+            const int r = i / CH, c = i % CH;
+            const bool ok = row0 + r < rows_end && c * 8 < P.D;
+            cp_async16_zfill(dst + r * PITCH + c * 16, src + (ok ? (long long)(row0 + r) * row_stride + c * 8 : 0), ok);
+        }
+    };
+    load_rows(q_sm, qg, P.qs[2], q0, P.Sq);
+    load_rows(kv_sm, kg, P.ks[2], k_begin, P.Skv);
+    load_rows(kv_sm + AM_BN * PITCH, vg, P.vs[2], k_begin, P.Skv);
+    cp_async_commit();
+
+    const int r0 = q0 + warp * 16 + (lane >> 2);  // this thread's rows: r0 and r0 + 8
+    const int cq = (lane & 3) * 2;                // column pair inside an 8-wide tile
+    const int lm_j = lane >> 3, lm_r = lane & 7;
+    const float c = P.scale * LOG2E;  // scale > 0
+    int first[2], last[2];            // keys each of the two rows may see
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const int qi = r0 + r * 8;
+        last[r] = causal ? min(P.Skv - 1, qi + offset) : P.Skv - 1;
+        first[r] = P.mask_kind == 4 ? qi + offset - P.window + 1 : 0;
+    }
+    const float* mask0 = P.mask + (ADD ? (P.mask_kind == 1 ? (long long)min(r0, P.Sq - 1) : (long long)b) * P.ms[0] : 0);
+    const long long mask_row8 = ADD && P.mask_kind == 1 ? (long long)(min(r0 + 8, P.Sq - 1) - min(r0, P.Sq - 1)) * P.ms[0] : 0;
+    uint32_t qa[DP / 16][4];
+    float o[DP / 8][4];
+#pragma unroll
+    for (int i = 0; i < DP / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
+    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.0f, 0.0f};
+
+    int buf = 0;
+    for (int kt = k_begin; kt < k_end; kt += AM_BN, buf ^= 1) {
+        cp_async_wait<0>();
+        __syncthreads();  // the tile is here, and everybody is done with the other buffer
+        if (kt + AM_BN < k_end) {
+            const uint32_t nx = kv_sm + (buf ^ 1) * 2 * AM_BN * PITCH;
+            load_rows(nx, kg, P.ks[2], kt + AM_BN, P.Skv);
+            load_rows(nx + AM_BN * PITCH, vg, P.vs[2], kt + AM_BN, P.Skv);
+            cp_async_commit();
+        }
+        if (kt == k_begin) {
+#pragma unroll
+            for (int ks = 0; ks < DP / 16; ++ks)
+                ldmatrix_x4(qa[ks], q_sm + (warp * 16 + (lm_j & 1) * 8 + lm_r) * PITCH + (ks * 2 + (lm_j >> 1)) * 16);
+        }
+        const uint32_t kb = kv_sm + buf * 2 * AM_BN * PITCH, vb = kb + AM_BN * PITCH;
+        // ---- S = Q K^T
+        float s[AM_BN / 8][4];
+#pragma unroll
+        for (int nt = 0; nt < AM_BN / 8; ++nt) {
+            s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.0f;
+#pragma unroll
+            for (int kp = 0; kp < DP / 32; ++kp) {
+                uint32_t bf[4];
+                ldmatrix_x4(bf, kb + (nt * 8 + lm_r) * PITCH + (kp * 4 + lm_j) * 16);
+                mma_16816<F16>(s[nt], qa[2 * kp], bf[0], bf[1]);
+                mma_16816<F16>(s[nt], qa[2 * kp + 1], bf[2], bf[3]);
+            }
+        }
+        // ---- log2 units; additive masks, then the tile's edges (causal diagonal, window, past the last key)
+        float2 c2 = make_float2(c, c);
+        if (ADD) {
+#pragma unroll
+            for (int nt = 0; nt < AM_BN / 8; ++nt) {
+                const int kj = kt + nt * 8 + cq;
+                const float* k0 = mask0 + (long long)min(kj, P.Skv - 1) * P.ms[1];
+                const float* k1 = mask0 + (long long)min(kj + 1, P.Skv - 1) * P.ms[1];
+                s[nt][0] = fmaf(__ldg(k0), LOG2E, s[nt][0] * c);
+                s[nt][1] = fmaf(__ldg(k1), LOG2E, s[nt][1] * c);
+                s[nt][2] = fmaf(__ldg(k0 + mask_row8), LOG2E, s[nt][2] * c);
+                s[nt][3] = fmaf(__ldg(k1 + mask_row8), LOG2E, s[nt][3] * c);
+            }
+            c2 = make_float2(1.0f, 1.0f);
+        }
+        if (kt + AM_BN > P.Skv || (causal && kt + AM_BN - 1 > q0 + warp * 16 + offset) ||
+            (P.mask_kind == 4 && kt + P.window <= q0 + warp * 16 + 15 + offset)) {
+#pragma unroll
+            for (int nt = 0; nt < AM_BN / 8; ++nt)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int kj = kt + nt * 8 + cq + (e & 1);
+                    if (kj > last[e >> 1] || kj < first[e >> 1]) s[nt][e] = -INFINITY;
+                }
+        }
+        // ---- online softmax; a row lives in the four threads of a quad.  m is the row maximum in log2 units.
+        float alpha[2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) am_softmax_row<AM_BN, ADD>(s, r, c, c2, m[r], l[r], alpha[r]);
+        // ---- O = O alpha + P V.  The tile's product is summed by itself: the tensor core cuts off what lies below its running
+        // sum, which over thousands of keys would show against f32 arithmetic; the sum over tiles is rounded properly.
+        float t[DP / 8][4];
+#pragma unroll
+        for (int i = 0; i < DP / 8; ++i) t[i][0] = t[i][1] = t[i][2] = t[i][3] = 0.0f;
+#pragma unroll
+        for (int kk = 0; kk < AM_BN / 16; ++kk) {
+            uint32_t pa[TERMS][4];
+#pragma unroll
+            for (int i = 0; i < TERMS; ++i) {
+                pa[i][0] = split_pair<F16>(s[2 * kk][0], s[2 * kk][1]);
+                pa[i][1] = split_pair<F16>(s[2 * kk][2], s[2 * kk][3]);
+                pa[i][2] = split_pair<F16>(s[2 * kk + 1][0], s[2 * kk + 1][1]);
+                pa[i][3] = split_pair<F16>(s[2 * kk + 1][2], s[2 * kk + 1][3]);
+            }
+#pragma unroll
+            for (int nd = 0; nd < DP / 16; ++nd) {
+                uint32_t bf[4];
+                ldmatrix_x4_trans(bf, vb + (kk * 16 + (lm_j & 1) * 8 + lm_r) * PITCH + (nd * 2 + (lm_j >> 1)) * 16);
+#pragma unroll
+                for (int i = TERMS - 1; i >= 0; --i) {
+                    mma_16816<F16>(t[2 * nd], pa[i], bf[0], bf[1]);
+                    mma_16816<F16>(t[2 * nd + 1], pa[i], bf[2], bf[3]);
+                }
+            }
+        }
+        am_accumulate<DP>(o, t, alpha);
+    }
+    am_store<DP>(P, o, l, r0, cq, b, h);
+}
+
+}  // namespace fusor

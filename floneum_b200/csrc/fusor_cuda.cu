@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "../../include/fusor_cuda.h"
+#include "attn_mma16.cuh"
 #include "decode_splitkv.cuh"
 #include "general_attention.cuh"
 #include "prefill_sm100.cuh"
@@ -157,6 +158,14 @@ extern "C" int32_t fusor_cuda_ctx_create(int32_t device, void* stream, fusor_cud
         {(const void*)oproj_sm100_kernel, (int)OP_SMEM_BYTES, "oproj_sm100_kernel"},
         {(const void*)decode_splitkv_kernel<128>, 227 * 1024, "decode_splitkv_kernel<128>"},
         {(const void*)decode_splitkv_kernel<64>, 227 * 1024, "decode_splitkv_kernel<64>"},
+        {(const void*)attn_mma16_kernel<96, false, false>, (int)am_smem_bytes<96>, "attn_mma16_kernel<96>"},
+        {(const void*)attn_mma16_kernel<96, false, true>, (int)am_smem_bytes<96>, "attn_mma16_kernel<96>"},
+        {(const void*)attn_mma16_kernel<96, true, false>, (int)am_smem_bytes<96>, "attn_mma16_kernel<96>"},
+        {(const void*)attn_mma16_kernel<96, true, true>, (int)am_smem_bytes<96>, "attn_mma16_kernel<96>"},
+        {(const void*)attn_mma16_kernel<128, false, false>, (int)am_smem_bytes<128>, "attn_mma16_kernel<128>"},
+        {(const void*)attn_mma16_kernel<128, false, true>, (int)am_smem_bytes<128>, "attn_mma16_kernel<128>"},
+        {(const void*)attn_mma16_kernel<128, true, false>, (int)am_smem_bytes<128>, "attn_mma16_kernel<128>"},
+        {(const void*)attn_mma16_kernel<128, true, true>, (int)am_smem_bytes<128>, "attn_mma16_kernel<128>"},
         {(const void*)general_attention_kernel, (int)general_smem_bytes(GEN_MAX_D), "general_attention_kernel"},
     };
     for (const auto& o : opt_in) {
@@ -409,6 +418,53 @@ static bool prefill_eligible(const AttnShape& S, const fusor_cuda_tensor4* q, co
     return true;
 }
 
+// Tensors of one type whose rows allow 16-byte loads and whose output rows allow paired stores.
+static bool mma_eligible(const AttnShape& S, const fusor_cuda_tensor4* q, const fusor_cuda_tensor4* k, const fusor_cuda_tensor4* v,
+                           float scale, const fusor_cuda_tensor4* out) {
+    if (S.D % 8 != 0 || S.D > 128 || !(scale > 0.0f) || !std::isfinite(scale)) return false;
+    if (q->dtype == FUSOR_CUDA_F32 || q->dtype != k->dtype || q->dtype != v->dtype) return false;
+    const int per16 = q->dtype == FUSOR_CUDA_F32 ? 4 : 8;
+    for (const fusor_cuda_tensor4* t : {q, k, v}) {
+        if (reinterpret_cast<uintptr_t>(t->data) % 16) return false;
+        for (int i = 0; i < 3; ++i)
+            if (t->shape[i] > 1 && t->stride[i] % per16 != 0) return false;
+    }
+    if (reinterpret_cast<uintptr_t>(out->data) % 8) return false;
+    for (int i = 0; i < 3; ++i)
+        if (out->shape[i] > 1 && out->stride[i] % 2 != 0) return false;
+    return true;
+}
+
+static int32_t launch_mma(fusor_cuda_ctx* ctx, const AttnShape& S, const fusor_cuda_tensor4* q, const fusor_cuda_tensor4* k,
+                            const fusor_cuda_tensor4* v, float scale, const fusor_cuda_tensor2* mask, int32_t mask_kind, int32_t window,
+                            const fusor_cuda_tensor4* out) {
+    AttnMmaParams P;
+    P.q = q->data; P.k = k->data; P.v = v->data; P.out = out->data; P.out_dtype = out->dtype;
+    P.mask = (mask_kind == FUSOR_CUDA_MASK_QK || mask_kind == FUSOR_CUDA_MASK_BATCH_KEY) ? (const float*)mask->data : nullptr;
+    P.B = S.B; P.Hq = S.Hq; P.Hkv = S.Hkv; P.Sq = S.Sq; P.Skv = S.Skv; P.D = S.D;
+    for (int i = 0; i < 3; ++i) {
+        P.qs[i] = q->stride[i]; P.ks[i] = k->stride[i]; P.vs[i] = v->stride[i]; P.os[i] = out->stride[i];
+    }
+    P.ms[0] = P.mask ? mask->stride[0] : 0;
+    P.ms[1] = P.mask ? mask->stride[1] : 0;
+    P.mask_kind = mask_kind; P.window = window; P.scale = scale;
+    P.n_q_tiles = (S.Sq + AM_BM - 1) / AM_BM;
+    const long long grid = (long long)P.n_q_tiles * S.Hq * S.B;
+    if (grid > 0x7fffffffLL) return fail(ctx, FUSOR_CUDA_UNSUPPORTED, "grid too large");
+    auto run = [&](auto bf16, auto bf16_add, auto f16, auto f16_add, size_t smem) {
+        auto kernel = q->dtype == FUSOR_CUDA_F16 ? (P.mask ? f16_add : f16) : (P.mask ? bf16_add : bf16);
+        kernel<<<(unsigned)grid, AM_THREADS, smem, ctx->stream>>>(P);
+    };
+#define FUSOR_AM(DP) run(attn_mma16_kernel<DP, false, false>, attn_mma16_kernel<DP, false, true>, attn_mma16_kernel<DP, true, false>, \
+                         attn_mma16_kernel<DP, true, true>, am_smem_bytes<DP>)
+    if (S.D <= 32) FUSOR_AM(32);
+    else if (S.D <= 64) FUSOR_AM(64);
+    else if (S.D <= 96) FUSOR_AM(96);
+    else FUSOR_AM(128);
+#undef FUSOR_AM
+    return launch_check(ctx, "attn_mma16_kernel");
+}
+
 // The softmax weights are kept in f16 against an f16 copy of V (the kernels fall back to bf16 weights and the bf16 V on
 // the device when some |v| does not fit f16).
 static int32_t launch_prefill(fusor_cuda_ctx* ctx, const AttnShape& S, const fusor_cuda_tensor4* q,
@@ -490,6 +546,7 @@ extern "C" int32_t fusor_cuda_flash_attention(fusor_cuda_ctx* ctx, const fusor_c
         return launch_prefill(ctx, S, q, k, v, scale, mask_kind, out, window,
                               mask_kind == FUSOR_CUDA_MASK_BATCH_KEY ? mask : nullptr,
                               mask_kind == FUSOR_CUDA_MASK_QK ? mask : nullptr);
+    if (mma_eligible(S, q, k, v, scale, out)) return launch_mma(ctx, S, q, k, v, scale, mask, mask_kind, window, out);
     return launch_general(ctx, S, q, k, v, scale, mask, mask_kind, window, out);
 }
 
