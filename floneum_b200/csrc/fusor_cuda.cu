@@ -22,6 +22,7 @@
 
 #include "../../include/fusor_cuda.h"
 #include "attn_mma16.cuh"
+#include "attn_mma32.cuh"
 #include "decode_splitkv.cuh"
 #include "general_attention.cuh"
 #include "prefill_sm100.cuh"
@@ -166,6 +167,14 @@ extern "C" int32_t fusor_cuda_ctx_create(int32_t device, void* stream, fusor_cud
         {(const void*)attn_mma16_kernel<128, false, true>, (int)am_smem_bytes<128>, "attn_mma16_kernel<128>"},
         {(const void*)attn_mma16_kernel<128, true, false>, (int)am_smem_bytes<128>, "attn_mma16_kernel<128>"},
         {(const void*)attn_mma16_kernel<128, true, true>, (int)am_smem_bytes<128>, "attn_mma16_kernel<128>"},
+        {(const void*)attn_mma32_kernel<32, false>, (int)a3_smem_bytes<32>, "attn_mma32_kernel<32>"},
+        {(const void*)attn_mma32_kernel<32, true>, (int)a3_smem_bytes<32>, "attn_mma32_kernel<32>"},
+        {(const void*)attn_mma32_kernel<64, false>, (int)a3_smem_bytes<64>, "attn_mma32_kernel<64>"},
+        {(const void*)attn_mma32_kernel<64, true>, (int)a3_smem_bytes<64>, "attn_mma32_kernel<64>"},
+        {(const void*)attn_mma32_kernel<96, false>, (int)a3_smem_bytes<96>, "attn_mma32_kernel<96>"},
+        {(const void*)attn_mma32_kernel<96, true>, (int)a3_smem_bytes<96>, "attn_mma32_kernel<96>"},
+        {(const void*)attn_mma32_kernel<128, false>, (int)a3_smem_bytes<128>, "attn_mma32_kernel<128>"},
+        {(const void*)attn_mma32_kernel<128, true>, (int)a3_smem_bytes<128>, "attn_mma32_kernel<128>"},
         {(const void*)general_attention_kernel, (int)general_smem_bytes(GEN_MAX_D), "general_attention_kernel"},
     };
     for (const auto& o : opt_in) {
@@ -422,7 +431,7 @@ static bool prefill_eligible(const AttnShape& S, const fusor_cuda_tensor4* q, co
 static bool mma_eligible(const AttnShape& S, const fusor_cuda_tensor4* q, const fusor_cuda_tensor4* k, const fusor_cuda_tensor4* v,
                            float scale, const fusor_cuda_tensor4* out) {
     if (S.D % 8 != 0 || S.D > 128 || !(scale > 0.0f) || !std::isfinite(scale)) return false;
-    if (q->dtype == FUSOR_CUDA_F32 || q->dtype != k->dtype || q->dtype != v->dtype) return false;
+    if (q->dtype != k->dtype || q->dtype != v->dtype) return false;
     const int per16 = q->dtype == FUSOR_CUDA_F32 ? 4 : 8;
     for (const fusor_cuda_tensor4* t : {q, k, v}) {
         if (reinterpret_cast<uintptr_t>(t->data) % 16) return false;
@@ -455,6 +464,14 @@ static int32_t launch_mma(fusor_cuda_ctx* ctx, const AttnShape& S, const fusor_c
         auto kernel = q->dtype == FUSOR_CUDA_F16 ? (P.mask ? f16_add : f16) : (P.mask ? bf16_add : bf16);
         kernel<<<(unsigned)grid, AM_THREADS, smem, ctx->stream>>>(P);
     };
+    if (q->dtype == FUSOR_CUDA_F32) {
+        auto run32 = [&](auto plain, auto add, size_t smem) { (P.mask ? add : plain)<<<(unsigned)grid, AM_THREADS, smem, ctx->stream>>>(P); };
+        if (S.D <= 32) run32(attn_mma32_kernel<32, false>, attn_mma32_kernel<32, true>, a3_smem_bytes<32>);
+        else if (S.D <= 64) run32(attn_mma32_kernel<64, false>, attn_mma32_kernel<64, true>, a3_smem_bytes<64>);
+        else if (S.D <= 96) run32(attn_mma32_kernel<96, false>, attn_mma32_kernel<96, true>, a3_smem_bytes<96>);
+        else run32(attn_mma32_kernel<128, false>, attn_mma32_kernel<128, true>, a3_smem_bytes<128>);
+        return launch_check(ctx, "attn_mma32_kernel");
+    }
 #define FUSOR_AM(DP) run(attn_mma16_kernel<DP, false, false>, attn_mma16_kernel<DP, false, true>, attn_mma16_kernel<DP, true, false>, \
                          attn_mma16_kernel<DP, true, true>, am_smem_bytes<DP>)
     if (S.D <= 32) FUSOR_AM(32);

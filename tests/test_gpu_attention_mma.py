@@ -60,3 +60,8 @@ SHAPES = [
 @pytest.mark.parametrize("dtype,out_dtype", [(1, 0), (2, 2)])
 def test_16_bit_tensors(device, dtype, out_dtype, shape):
     _case(device, dtype, out_dtype, *shape)
+
+
+@pytest.mark.parametrize("shape", SHAPES + [(2, 2, 1, 64, 95, 128, "causal"), (1, 2, 2, 33, 33, 128, "window"), (2, 2, 1, 31, 32, 8, "key")])
+def test_f32_tensors(device, shape):
+    _case(device, 0, 0, *shape)
