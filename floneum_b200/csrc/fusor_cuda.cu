@@ -175,7 +175,18 @@ extern "C" int32_t fusor_cuda_ctx_create(int32_t device, void* stream, fusor_cud
         {(const void*)attn_mma32_kernel<96, true>, (int)a3_smem_bytes<96>, "attn_mma32_kernel<96>"},
         {(const void*)attn_mma32_kernel<128, false>, (int)a3_smem_bytes<128>, "attn_mma32_kernel<128>"},
         {(const void*)attn_mma32_kernel<128, true>, (int)a3_smem_bytes<128>, "attn_mma32_kernel<128>"},
-        {(const void*)general_attention_kernel, (int)general_smem_bytes(GEN_MAX_D), "general_attention_kernel"},
+        {(const void*)general_attention_kernel<8, 1, true>, (int)general_smem_bytes(64, 8), "general_attention_kernel<8, 1>"},
+        {(const void*)general_attention_kernel<8, 1, false>, (int)general_smem_bytes(64, 8), "general_attention_kernel<8, 1>"},
+        {(const void*)general_attention_kernel<4, 1, true>, (int)general_smem_bytes(64, 4), "general_attention_kernel<4, 1>"},
+        {(const void*)general_attention_kernel<4, 1, false>, (int)general_smem_bytes(64, 4), "general_attention_kernel<4, 1>"},
+        {(const void*)general_attention_kernel<8, 2, true>, (int)general_smem_bytes(128, 8), "general_attention_kernel<8, 2>"},
+        {(const void*)general_attention_kernel<8, 2, false>, (int)general_smem_bytes(128, 8), "general_attention_kernel<8, 2>"},
+        {(const void*)general_attention_kernel<4, 2, true>, (int)general_smem_bytes(128, 4), "general_attention_kernel<4, 2>"},
+        {(const void*)general_attention_kernel<4, 2, false>, (int)general_smem_bytes(128, 4), "general_attention_kernel<4, 2>"},
+        {(const void*)general_attention_kernel<4, 3, true>, (int)general_smem_bytes(192, 4), "general_attention_kernel<4, 3>"},
+        {(const void*)general_attention_kernel<4, 3, false>, (int)general_smem_bytes(192, 4), "general_attention_kernel<4, 3>"},
+        {(const void*)general_attention_kernel<4, 4, true>, (int)general_smem_bytes(256, 4), "general_attention_kernel<4, 4>"},
+        {(const void*)general_attention_kernel<4, 4, false>, (int)general_smem_bytes(256, 4), "general_attention_kernel<4, 4>"},
     };
     for (const auto& o : opt_in) {
         cudaError_t e = cudaFuncSetAttribute(o.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, o.bytes);
@@ -370,9 +381,26 @@ static int32_t launch_general(fusor_cuda_ctx* ctx, const AttnShape& S, const fus
     P.ms[0] = P.mask ? mask->stride[0] : 0;
     P.ms[1] = P.mask ? mask->stride[1] : 0;
     P.mask_kind = mask_kind; P.window = window; P.scale = scale;
-    if (S.Hq > 65535 || S.B > 65535) return fail(ctx, FUSOR_CUDA_UNSUPPORTED, "more than 65535 heads or batches");
-    dim3 grid((S.Sq + GEN_BM - 1) / GEN_BM, S.Hq, S.B);
-    general_attention_kernel<<<grid, GEN_THREADS, general_smem_bytes(S.D), ctx->stream>>>(P);
+    bool vec = q->dtype == FUSOR_CUDA_F32 && k->dtype == FUSOR_CUDA_F32 && v->dtype == FUSOR_CUDA_F32 && S.D % 4 == 0;
+    for (const fusor_cuda_tensor4* t : {q, k, v, out}) {
+        vec = vec && reinterpret_cast<uintptr_t>(t->data) % 16 == 0;
+        for (int i = 0; i < 3; ++i) vec = vec && (t->shape[i] == 1 || t->stride[i] % 4 == 0);
+    }
+    const int nc = (S.D + 63) / 64;
+    const long long tiles64 = (long long)((S.Sq + 63) / 64) * S.Hq * S.B;
+    const int rt = nc <= 2 && tiles64 >= 3ll * ctx->num_sms ? 8 : 4;
+    P.n_q_tiles = (S.Sq + 8 * rt - 1) / (8 * rt);
+    const long long grid = (long long)P.n_q_tiles * S.Hq * S.B;
+    if (grid > 0x7fffffffLL) return fail(ctx, FUSOR_CUDA_UNSUPPORTED, "grid too large");
+    auto run = [&](auto kernel_vec, auto kernel) {
+        (vec ? kernel_vec : kernel)<<<(unsigned)grid, GEN_THREADS, general_smem_bytes(S.D, rt), ctx->stream>>>(P);
+    };
+    if (nc == 1) rt == 8 ? run(general_attention_kernel<8, 1, true>, general_attention_kernel<8, 1, false>)
+                         : run(general_attention_kernel<4, 1, true>, general_attention_kernel<4, 1, false>);
+    else if (nc == 2) rt == 8 ? run(general_attention_kernel<8, 2, true>, general_attention_kernel<8, 2, false>)
+                              : run(general_attention_kernel<4, 2, true>, general_attention_kernel<4, 2, false>);
+    else if (nc == 3) run(general_attention_kernel<4, 3, true>, general_attention_kernel<4, 3, false>);
+    else run(general_attention_kernel<4, 4, true>, general_attention_kernel<4, 4, false>);
     return launch_check(ctx, "general_attention_kernel");
 }
 
