@@ -53,6 +53,7 @@ struct fusor_cuda_ctx {
     size_t v16_bytes = 0;
     int* d_flags = nullptr;  // [256]
     unsigned flag_counter = 0;
+    int clusters[4] = {};  // clusters of 1, 2, 4, 8 CTAs that can be resident at once, one CTA per SM
     // copy streams of the _host entry points (host -> device, device -> host), created on first use
     cudaStream_t h2d_stream = nullptr, d2h_stream = nullptr;
 };
@@ -109,6 +110,20 @@ extern "C" int32_t fusor_cuda_device_count(int32_t* count) {
     return FUSOR_CUDA_OK;
 }
 
+static cudaLaunchConfig_t cluster_config(const fusor_cuda_ctx* ctx, unsigned ctas, unsigned cluster, unsigned threads, size_t smem,
+                                         cudaLaunchAttribute* attr) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas, 1, 1);
+    cfg.blockDim = dim3(threads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = cluster; attr->val.clusterDim.y = 1; attr->val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
 extern "C" int32_t fusor_cuda_ctx_create(int32_t device, void* stream, fusor_cuda_ctx** out) {
     if (!out) return fail(nullptr, FUSOR_CUDA_INVALID_ARGUMENT, "out is null");
     *out = nullptr;
@@ -156,7 +171,8 @@ extern "C" int32_t fusor_cuda_ctx_create(int32_t device, void* stream, fusor_cud
     struct { const void* fn; int bytes; const char* name; } opt_in[] = {
         {(const void*)prefill_sm100_kernel, (int)PF_SMEM_BYTES, "prefill_sm100_kernel"},
         {(const void*)prefill2_sm100_kernel, (int)P2_SMEM_BYTES, "prefill2_sm100_kernel"},
-        {(const void*)oproj_sm100_kernel, (int)OP_SMEM_BYTES, "oproj_sm100_kernel"},
+        {(const void*)oproj_pair_kernel, (int)OP2_SMEM_BYTES, "oproj_pair_kernel"},
+        {(const void*)oproj_split_kernel, (int)OPS_SMEM_BYTES, "oproj_split_kernel"},
         {(const void*)decode_splitkv_kernel<128>, 227 * 1024, "decode_splitkv_kernel<128>"},
         {(const void*)decode_splitkv_kernel<64>, 227 * 1024, "decode_splitkv_kernel<64>"},
         {(const void*)attn_mma16_kernel<96, false, false>, (int)am_smem_bytes<96>, "attn_mma16_kernel<96>"},
@@ -194,6 +210,16 @@ extern "C" int32_t fusor_cuda_ctx_create(int32_t device, void* stream, fusor_cud
             cudaGetLastError();
             fusor_cuda_ctx_destroy(ctx);
             return fail(nullptr, FUSOR_CUDA_CUDA_ERROR, "shared memory opt-in of %s (%d bytes): %s", o.name, o.bytes, cudaGetErrorString(e));
+        }
+    }
+    // a cluster needs its SMs in one GPC, so fewer clusters fit than SMs / size
+    ctx->clusters[0] = ctx->num_sms;
+    for (int i = 1; i < 4; ++i) {
+        cudaLaunchAttribute attr;
+        cudaLaunchConfig_t cfg = cluster_config(ctx, (ctx->num_sms >> i) << i, 1 << i, OP_THREADS, OPS_SMEM_BYTES, &attr);
+        if (cudaOccupancyMaxActiveClusters(&ctx->clusters[i], oproj_split_kernel, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            ctx->clusters[i] = 0;
         }
     }
     *out = ctx;
@@ -606,6 +632,42 @@ extern "C" int32_t fusor_cuda_flash_attention_general(fusor_cuda_ctx* ctx, const
 }
 
 // --------------------------------------------------------------------------- output projection
+// Which of the three kernels: by the number of output tiles, see oproj_sm100.cuh.
+static int32_t launch_out_proj(fusor_cuda_ctx* ctx, const fusor_cuda_tensor4* attn, const fusor_cuda_tensor4* w4,
+                               const fusor_cuda_tensor4* out, OprojParams& P) {
+    const long long rows = (long long)P.B * P.S, K = (long long)P.k_chunks * OP_BK;
+    if (rows <= OPR_MAX_ROWS) {
+        const unsigned blocks = (unsigned)((P.N + 15) / 16);
+        if (rows <= 8) oproj_rows_kernel<1><<<blocks, OPR_WARPS * 32, 0, ctx->stream>>>(P);
+        else oproj_rows_kernel<2><<<blocks, OPR_WARPS * 32, 0, ctx->stream>>>(P);
+        return launch_check(ctx, "oproj_rows_kernel");
+    }
+    const long long m_tiles = (long long)P.B * P.m_tiles_per_batch;
+    CUtensorMap tmA, tmW, tmO;
+    TRY(make_tmap_bhsd(ctx, &tmA, attn, OP_BM));
+    TRY(make_tmap_bhsd(ctx, &tmW, w4, 128));
+    const long long tiles128 = m_tiles * ((P.N + OPS_BN - 1) / OPS_BN);
+    if (tiles128 <= ctx->num_sms) {
+        P.n_tiles = (P.N + OPS_BN - 1) / OPS_BN;
+        // as many CTAs per tile as fit at once, each with at least four K steps (a full ring)
+        int i = 0;
+        while ((2 << i) <= OPS_MAX_SPLIT && tiles128 <= ctx->clusters[i + 1] && P.k_chunks >= 4 * (2 << i)) ++i;
+        const int ks = 1 << i;
+        cudaLaunchAttribute attr;
+        const cudaLaunchConfig_t cfg = cluster_config(ctx, (unsigned)(tiles128 * ks), (unsigned)ks, OP_THREADS, OPS_SMEM_BYTES, &attr);
+        CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, oproj_split_kernel, tmA, tmW, P, ks));
+        return launch_check(ctx, "oproj_split_kernel");
+    }
+    TRY(make_tmap_bhsd(ctx, &tmO, out, 32, tmap_dtype(out->dtype)));
+    P.n_tiles = (P.N + OP2_BN - 1) / OP2_BN;
+    P.n_group = (int)std::max<long long>(1, std::min<long long>(P.n_tiles, (32ll << 20) / ((long long)OP2_BN * K * 2)));
+    const long long tiles = (m_tiles + 1) / 2 * P.n_tiles;
+    if (tiles > 0x7fffffffLL) return fail(ctx, FUSOR_CUDA_UNSUPPORTED, "too many output tiles");
+    const unsigned pairs = (unsigned)std::min<long long>(tiles, ctx->num_sms / 2);  // persistent: one CTA pair per two SMs
+    oproj_pair_kernel<<<2 * pairs, OP_THREADS, OP2_SMEM_BYTES, ctx->stream>>>(tmA, tmW, tmO, P);
+    return launch_check(ctx, "oproj_pair_kernel");
+}
+
 extern "C" int32_t fusor_cuda_attention_out_proj(fusor_cuda_ctx* ctx, const fusor_cuda_tensor4* attn,
                                                  const fusor_cuda_tensor4* weight, const float* bias,
                                                  const fusor_cuda_tensor4* out) {
@@ -633,22 +695,16 @@ extern "C" int32_t fusor_cuda_attention_out_proj(fusor_cuda_ctx* ctx, const fuso
     DeviceGuard g(ctx->device);
     fusor_cuda_tensor4 w4 = *weight;
     w4.stride[0] = w4.stride[1] = N * weight->stride[2];
-    CUtensorMap tmA, tmW, tmO;
-    TRY(make_tmap_bhsd(ctx, &tmA, attn, OP_BM));
-    TRY(make_tmap_bhsd(ctx, &tmW, &w4, OP_BN));
-    TRY(make_tmap_bhsd(ctx, &tmO, out, 32, tmap_dtype(out->dtype)));
-    OprojParams P;
+    OprojParams P{};
     P.B = (int)B; P.Hq = (int)Hq; P.S = (int)S; P.D = (int)D; P.N = (int)N;
     P.m_tiles_per_batch = (int)((S + OP_BM - 1) / OP_BM);
-    P.n_tiles = (int)((N + OP_BN - 1) / OP_BN);
     P.k_chunks = (int)(K / OP_BK);
-    P.n_group = (int)std::max<long long>(1, std::min<long long>(P.n_tiles, (32ll << 20) / ((long long)OP_BN * K * 2)));
     P.bias = bias; P.out_dtype = out->dtype; P.err = ctx->d_err;
-    const long long tiles = B * P.m_tiles_per_batch * P.n_tiles;
-    if (tiles > 0x7fffffffLL) return fail(ctx, FUSOR_CUDA_UNSUPPORTED, "too many output tiles");
-    const unsigned ctas = (unsigned)std::min<long long>(tiles, ctx->num_sms);
-    oproj_sm100_kernel<<<ctas, OP_THREADS, OP_SMEM_BYTES, ctx->stream>>>(tmA, tmW, tmO, P);
-    return launch_check(ctx, "oproj_sm100_kernel");
+    P.a = static_cast<const __nv_bfloat16*>(attn->data);
+    for (int i = 0; i < 3; ++i) P.as[i] = attn->stride[i];
+    P.w = static_cast<const __nv_bfloat16*>(weight->data); P.ws = weight->stride[2];
+    P.out = out->data; P.os[0] = out->stride[0]; P.os[1] = out->stride[2];
+    return launch_out_proj(ctx, attn, &w4, out, P);
 }
 
 // --------------------------------------------------------------------------- host-memory variants
