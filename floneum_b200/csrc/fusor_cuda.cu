@@ -15,9 +15,11 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <string>
 #include <thread>
+#include <unordered_map>
 #include <vector>
 
 #include "../../include/fusor_cuda.h"
@@ -33,6 +35,136 @@
 
 using namespace fusor;
 
+// =============================================================================== device buffers kept for reuse
+// Buffers of fusor_cuda_buffer_alloc / _free.  Every call of the host mirrors allocates its result, and a cudaMalloc +
+// cudaFree pair with the device-wide wait inside cudaFree cost 0.4 to 3 ms of host time, many times the kernels (back to back:
+// attention of a 777-token prompt 0.8 to 3 ms, 29 us with kept buffers; a prefill of B4 S4096 with its 268 MB result 1.5 ms
+// and 0.60 ms).  A freed buffer may still be read by work on ANY stream (the library's, torch's), which is why cudaFree waits
+// for the whole device; here freed buffers wait together: they are handed out again only after a cudaDeviceSynchronize that
+// came after their release.  That wait is made when a buffer of the size is among them and the context's own stream has
+// nothing to do (a program that reads its results back is there already), or enough of the size are waiting to spread its
+// cost.  Kept: at most a 64th of the device's memory; larger buffers than a quarter of that go straight to cudaMalloc /
+// cudaFree, and so does everything while the context's stream is being captured (a graph keeps the addresses it saw).
+class BufferPool {
+  public:
+    void set_limit(size_t bytes) { limit_ = bytes; }
+
+    cudaError_t alloc(size_t bytes, cudaStream_t stream, void** out) {
+        const size_t size = rounded(bytes);
+        if (size > limit_ / 4) return plain(bytes, out);
+        std::lock_guard<std::mutex> lock(mutex_);
+        if (take(size, out)) return cudaSuccess;
+        auto waiting = freed_of_.find(size);
+        if (waiting != freed_of_.end()) {
+            bool now = waiting->second >= std::max<size_t>(8, std::min<size_t>(256, (64u << 20) / size));
+            if (!now) {
+                now = cudaStreamQuery(stream) == cudaSuccess;
+                if (!now) cudaGetLastError();  // not ready
+            }
+            if (now) {
+                const cudaError_t e = settle();
+                if (e != cudaSuccess) return e;
+                if (take(size, out)) return cudaSuccess;
+            }
+        }
+        cudaError_t e = cudaMalloc(out, size);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            if (settle() == cudaSuccess) trim(0);
+            e = cudaMalloc(out, size);
+        }
+        if (e == cudaSuccess) live_[*out] = size;
+        return e;
+    }
+
+    enum Release { KEPT, NOT_KEPT, FREED_TWICE };
+    // KEPT: the buffer is kept for reuse.  NOT_KEPT: the caller gives it to cudaFree (not one of the pool's, or the pool is
+    // full); the pool has forgotten it.
+    Release release(void* p) {
+        std::lock_guard<std::mutex> lock(mutex_);
+        auto it = live_.find(p);
+        if (it == live_.end()) {
+            for (const Block& b : freed_)
+                if (b.ptr == p) return FREED_TWICE;
+            for (const auto& b : ready_)
+                if (b.second == p) return FREED_TWICE;
+            return NOT_KEPT;
+        }
+        const size_t size = it->second;
+        live_.erase(it);
+        if (kept_ + size > limit_) {
+            if (settle() == cudaSuccess) trim(limit_ / 2);
+            if (kept_ + size > limit_) return NOT_KEPT;
+        }
+        freed_.push_back({p, size});
+        ++freed_of_[size];
+        kept_ += size;
+        return KEPT;
+    }
+
+    // cudaMalloc for the library's own workspaces: what the pool keeps must not be the reason that one fails
+    cudaError_t plain(size_t bytes, void** out) {
+        cudaError_t e = cudaMalloc(out, bytes);
+        if (e == cudaErrorMemoryAllocation) {
+            std::lock_guard<std::mutex> lock(mutex_);
+            if (kept_ == 0) return e;
+            cudaGetLastError();
+            if (settle() == cudaSuccess) trim(0);
+            e = cudaMalloc(out, bytes);
+        }
+        return e;
+    }
+
+    void drain() {  // gives everything kept back
+        std::lock_guard<std::mutex> lock(mutex_);
+        if (kept_ > 0 && settle() == cudaSuccess) trim(0);
+    }
+
+  private:
+    struct Block {
+        void* ptr;
+        size_t size;
+    };
+    // sizes that repeat are found again; the slack is at most an eighth
+    static size_t rounded(size_t bytes) {
+        size_t unit = 512;
+        while (unit * 16 <= bytes) unit *= 2;
+        return (std::max<size_t>(bytes, 1) + unit - 1) / unit * unit;
+    }
+    bool take(size_t size, void** out) {
+        auto it = ready_.lower_bound(size);
+        if (it == ready_.end() || it->first > size + size / 4) return false;
+        *out = it->second;
+        live_[it->second] = it->first;
+        kept_ -= it->first;
+        ready_.erase(it);
+        return true;
+    }
+    cudaError_t settle() {
+        const cudaError_t e = cudaDeviceSynchronize();
+        if (e != cudaSuccess) return e;
+        for (const Block& b : freed_) ready_.emplace(b.size, b.ptr);
+        freed_.clear();
+        freed_of_.clear();
+        return cudaSuccess;
+    }
+    void trim(size_t target) {  // cudaFree of ready buffers, largest first
+        while (kept_ > target && !ready_.empty()) {
+            auto it = std::prev(ready_.end());
+            cudaFree(it->second);
+            kept_ -= it->first;
+            ready_.erase(it);
+        }
+    }
+
+    std::mutex mutex_;
+    size_t limit_ = 0, kept_ = 0;
+    std::unordered_map<void*, size_t> live_;       // handed out
+    std::vector<Block> freed_;                     // released since the last device-wide wait
+    std::unordered_map<size_t, size_t> freed_of_;  // how many of a size
+    std::multimap<size_t, void*> ready_;           // released before it
+};
+
 // =============================================================================== context
 struct fusor_cuda_ctx {
     int device = 0;
@@ -42,6 +174,7 @@ struct fusor_cuda_ctx {
     int* d_err = nullptr;  // device error word written by kernels
     long long launches = 0;
     std::string last_error;
+    BufferPool pool;  // results and other buffers of fusor_cuda_buffer_alloc
     PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
     // scratch owned by the context for the _host entry points
     void* scratch = nullptr;
@@ -142,6 +275,7 @@ extern "C" int32_t fusor_cuda_ctx_create(int32_t device, void* stream, fusor_cud
     fusor_cuda_ctx* ctx = new fusor_cuda_ctx();
     ctx->device = device;
     ctx->num_sms = prop.multiProcessorCount;
+    ctx->pool.set_limit(prop.totalGlobalMem / 64);
     if (stream) {
         ctx->stream = static_cast<cudaStream_t>(stream);
     } else {
@@ -230,6 +364,7 @@ extern "C" int32_t fusor_cuda_ctx_destroy(fusor_cuda_ctx* ctx) {
     if (!ctx) return FUSOR_CUDA_OK;
     DeviceGuard g(ctx->device);
     cudaStreamSynchronize(ctx->stream);
+    ctx->pool.drain();
     if (ctx->scratch) cudaFree(ctx->scratch);
     if (ctx->pinned) cudaFreeHost(ctx->pinned);
     if (ctx->v16) cudaFree(ctx->v16);
@@ -285,15 +420,29 @@ extern "C" int32_t fusor_cuda_stream_sync(fusor_cuda_ctx* ctx) {
     return check_device_error(ctx);
 }
 
+static bool capturing(fusor_cuda_ctx* ctx) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &st) != cudaSuccess) {
+        cudaGetLastError();  // the legacy stream while another one captures
+        return true;
+    }
+    return st != cudaStreamCaptureStatusNone;
+}
+
 extern "C" int32_t fusor_cuda_buffer_alloc(fusor_cuda_ctx* ctx, size_t bytes, void** device_ptr) {
     if (!ctx || !device_ptr) return fail(ctx, FUSOR_CUDA_INVALID_ARGUMENT, "null argument");
     DeviceGuard g(ctx->device);
-    CUDA_TRY(ctx, cudaMalloc(device_ptr, bytes ? bytes : 1));
+    if (capturing(ctx)) CUDA_TRY(ctx, cudaMalloc(device_ptr, bytes ? bytes : 1));
+    else CUDA_TRY(ctx, ctx->pool.alloc(bytes ? bytes : 1, ctx->stream, device_ptr));
     return FUSOR_CUDA_OK;
 }
 extern "C" int32_t fusor_cuda_buffer_free(fusor_cuda_ctx* ctx, void* device_ptr) {
     if (!ctx) return fail(ctx, FUSOR_CUDA_INVALID_ARGUMENT, "ctx is null");
     DeviceGuard g(ctx->device);
+    if (capturing(ctx)) CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));  // refused, as cudaFree is
+    const BufferPool::Release r = ctx->pool.release(device_ptr);
+    if (r == BufferPool::KEPT) return FUSOR_CUDA_OK;
+    if (r == BufferPool::FREED_TWICE) return fail(ctx, FUSOR_CUDA_CUDA_ERROR, "the buffer has been freed already");
     CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
     CUDA_TRY(ctx, cudaFree(device_ptr));
     return FUSOR_CUDA_OK;
@@ -562,7 +711,7 @@ static int32_t launch_prefill(fusor_cuda_ctx* ctx, const AttnShape& S, const fus
             if (ctx->v16) CUDA_TRY(ctx, cudaFree(ctx->v16));
             ctx->v16 = nullptr;
             ctx->v16_bytes = 0;
-            CUDA_TRY(ctx, cudaMalloc(&ctx->v16, n * 2));
+            CUDA_TRY(ctx, ctx->pool.plain(n * 2, &ctx->v16));
             ctx->v16_bytes = n * 2;
         }
         const unsigned slot = ctx->flag_counter++ % 256;
@@ -716,7 +865,7 @@ static int32_t ensure_scratch(fusor_cuda_ctx* ctx, size_t bytes) {
         ctx->scratch = nullptr;
         ctx->scratch_bytes = 0;
     }
-    CUDA_TRY(ctx, cudaMalloc(&ctx->scratch, bytes));
+    CUDA_TRY(ctx, ctx->pool.plain(bytes, &ctx->scratch));
     ctx->scratch_bytes = bytes;
     return FUSOR_CUDA_OK;
 }
@@ -893,10 +1042,11 @@ extern "C" int32_t fusor_cuda_kvcache_create(fusor_cuda_ctx* ctx, int32_t max_ba
     const size_t pool_bytes = (size_t)num_pages * num_kv_heads * DEC_PT * head_dim * 2;
     c->max_grid = DEC_CTAS * ctx->num_sms;
     c->max_slots = max_batch * num_kv_heads + c->max_grid;
-    bool ok = cudaMalloc(&c->k_pages, pool_bytes) == cudaSuccess && cudaMalloc(&c->v_pages, pool_bytes) == cudaSuccess &&
-              cudaMalloc(&c->d_tables, ((size_t)2 * max_batch + (size_t)max_batch * max_pages_per_seq) * 4) == cudaSuccess &&
-              cudaMalloc(&c->part_o, (size_t)c->max_slots * DEC_GP * head_dim * 4) == cudaSuccess &&
-              cudaMalloc(&c->part_ml, (size_t)c->max_slots * DEC_GP * 2 * 4) == cudaSuccess;
+    auto alloc = [&](auto** p, size_t bytes) { return ctx->pool.plain(bytes, reinterpret_cast<void**>(p)); };
+    bool ok = alloc(&c->k_pages, pool_bytes) == cudaSuccess && alloc(&c->v_pages, pool_bytes) == cudaSuccess &&
+              alloc(&c->d_tables, ((size_t)2 * max_batch + (size_t)max_batch * max_pages_per_seq) * 4) == cudaSuccess &&
+              alloc(&c->part_o, (size_t)c->max_slots * DEC_GP * head_dim * 4) == cudaSuccess &&
+              alloc(&c->part_ml, (size_t)c->max_slots * DEC_GP * 2 * 4) == cudaSuccess;
     if (ok) {
         c->d_len_before = c->d_tables;
         c->d_kv_len = c->d_tables + max_batch;
@@ -1262,7 +1412,7 @@ extern "C" int32_t fusor_cuda_kvcache_truncate_front(fusor_cuda_kvcache* c, int3
             c->shift_buf = nullptr;
             c->shift_bytes = 0;
             const size_t want = 2 * align256((size_t)c->Hkv * c->max_pages * DEC_PT * c->D * 2);  // the longest sequence: no regrowth
-            CUDA_TRY(ctx, cudaMalloc(&c->shift_buf, want));
+            CUDA_TRY(ctx, ctx->pool.plain(want, reinterpret_cast<void**>(&c->shift_buf)));
             c->shift_bytes = want;
         }
         TRY(kv_sync_tables(c));
