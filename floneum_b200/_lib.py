@@ -82,6 +82,7 @@ SIGNATURES = {
     "fusor_cuda_rope": (c_int32, [c_void_p, _T4, c_void_p, c_void_p, c_int32, c_int32, c_int32, _T4]),
     "fusor_cuda_kvcache_rope_append": (c_int32, [c_void_p, _T4, _T4, _T4, c_void_p, c_void_p, c_int32, c_int32, c_int32, _T4]),
     "fusor_cuda_kvcache_truncate_front": (c_int32, [c_void_p, c_int32, c_int32]),
+    "fusor_cuda_kvcache_drop_front": (c_int32, [c_void_p, c_int32, c_int32]),
     "fusor_cuda_kvcache_seq_len": (c_int32, [c_void_p, c_int32, POINTER(c_int32)]),
     "fusor_cuda_kvcache_set_page_table": (c_int32, [c_void_p, POINTER(c_int32), POINTER(c_int32), c_int32]),
     "fusor_cuda_kvcache_write_pages": (c_int32, [c_void_p, c_int32, c_int32, c_void_p, c_void_p]),

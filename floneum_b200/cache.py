@@ -158,6 +158,10 @@ class PagedKvCache:
     def truncate_front(self, b: int, keep: int):
         self._ck(self._L.fusor_cuda_kvcache_truncate_front(self._h, b, keep))
 
+    def drop_front(self, b: int, keep: int):
+        """truncate_front without moving the kept rows: up to 15 evicted rows stay, skipped, in the first page."""
+        self._ck(self._L.fusor_cuda_kvcache_drop_front(self._h, b, keep))
+
     def seq_len(self, b: int = 0) -> int:
         n = ctypes.c_int32()
         self._ck(self._L.fusor_cuda_kvcache_seq_len(self._h, b, ctypes.byref(n)))
@@ -323,7 +327,7 @@ class KvCache:
             v = Tensor(device, v.ptr + skip * v.strides[2] * (4 if v.dtype == F32 else 2), (B, Hkv, mx, D), v.dtype, v.strides, owner=v)
         elif self.current_seq_len() + n > mx:
             for b in range(B):
-                self._paged.truncate_front(b, mx - n)
+                self._paged.drop_front(b, mx - n)
         return k, v, skip
 
     def append(self, device: Device, k: Tensor, v: Tensor) -> Tuple[CachedKv, CachedKv]:
@@ -358,6 +362,8 @@ class KvCache:
         if n == 0:
             z = np.zeros((self._batch, self._num_kv_heads, 0, self._head_dim), np.float32)
             return {"k": z, "v": z.copy(), "max_sequence_len": self.max_sequence_len}
+        for b in range(self._batch):  # the rows where an import will put them, so that both caches decode to the same bits
+            self._paged.truncate_front(b, n)
         k, v = self._dense(F32)
         return {"k": k.as_slice(), "v": v.as_slice(), "max_sequence_len": self.max_sequence_len}
 

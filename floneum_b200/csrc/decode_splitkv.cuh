@@ -121,7 +121,9 @@ struct DecodeParams {
     const int* page_table;
     int max_pages;
     int num_pages;
-    const int* kv_len;         // [B] device-resident lengths; a sequence may be empty when records are asked for (modes 1, 2)
+    const int* end;            // [B] device-resident: where each sequence's rows end, counted from its first page's first row
+    const int* front;          // [B] evicted rows at the start of the first page; an empty sequence (when records are asked
+                               // for, modes 1 and 2) has end = front = 0
     int B;
     float* part_o;             // [slots][DEC_GP][D], slots >= B * Hkv + grid
     float* part_ml;            // [slots][DEC_GP][2]  (m in log2 units, l)
@@ -201,7 +203,7 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS) decode_splitkv_kernel(c
         int sum = 0;
         for (int b0 = 0; b0 < P.B; b0 += 32) {
             const int b = b0 + lane;
-            int pg = b < P.B ? (P.kv_len[b] + DEC_PT - 1) / DEC_PT : 0;
+            int pg = b < P.B ? (P.end[b] + DEC_PT - 1) / DEC_PT : 0;
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) pg += __shfl_xor_sync(0xffffffffu, pg, o);
             sum += pg;
@@ -212,7 +214,7 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS) decode_splitkv_kernel(c
         int b_start = P.B;
         for (int b0 = 0; b0 < P.B; b0 += 32) {
             const int b = b0 + lane;
-            const int pg = b < P.B ? (P.kv_len[b] + DEC_PT - 1) / DEC_PT : 0;
+            const int pg = b < P.B ? (P.end[b] + DEC_PT - 1) / DEC_PT : 0;
             int incl = pg;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -250,7 +252,7 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS) decode_splitkv_kernel(c
         int slot = 0, phase = 0;  // ring position of the next page; `phase` flips each time the ring wraps
         bool wrapped = false;
         bool ok = true;
-        while (ok && decode_next_segment(P.kv_len, P.B, P.Hkv, T, (int)gridDim.x, (int)blockIdx.x, W, S)) {
+        while (ok && decode_next_segment(P.end, P.B, P.Hkv, T, (int)gridDim.x, (int)blockIdx.x, W, S)) {
             const int* pt = P.page_table + (long long)S.b * P.max_pages;
             int next_phys = (S.page_begin + lane < S.page_end) ? pt[S.page_begin + lane] : 0;
             for (int p0 = S.page_begin; p0 < S.page_end && ok; p0 += 32) {
@@ -303,15 +305,17 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS) decode_splitkv_kernel(c
             DecodeWalk w0;
             decode_walk_init(w0, T, (int)gridDim.x, (int)blockIdx.x, walk0[1], walk0[2]);
             DecodeSegment s0;
-            *have_seg = decode_next_segment(P.kv_len, P.B, P.Hkv, T, (int)gridDim.x, (int)blockIdx.x, w0, s0) ? 1 : 0;
+            *have_seg = decode_next_segment(P.end, P.B, P.Hkv, T, (int)gridDim.x, (int)blockIdx.x, w0, s0) ? 1 : 0;
             *walk_s = w0;
             *seg_s = s0;
         }
         named_bar_sync(1, NC);
         while (*have_seg) {
             // what the page loop needs of the segment; the rest is read again from shared memory afterwards
-            const int seg_page_begin = seg_s->page_begin, seg_off = seg_s->cta_page_off, seg_kv_len = seg_s->kv_len;
-            const int n_pages = seg_s->page_end - seg_page_begin;
+            const int seg_off = seg_s->cta_page_off, seg_last = seg_off + seg_s->page_end - seg_s->page_begin;
+            const int front = P.front[seg_s->b], seg_len = seg_s->kv_len - front;
+            // token 0 of page i of the CTA's stream, counted from the first row that has not been evicted
+            const int seg_tok = (seg_s->page_begin - seg_off) * DEC_PT - front;
             // Q fragments: rows >= g are zero.
             uint32_t qa[D / 16][2];
 #pragma unroll
@@ -343,7 +347,7 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS) decode_splitkv_kernel(c
             // has seen it (the owner: once it has used it).  The producer refills a slot only after all DEC_NW
             // releases, so no warp can meet a slot's barrier two phases later, which a parity wait cannot tell
             // from "ready".
-            for (int i = seg_off; i < seg_off + n_pages; ++i) {
+            for (int i = seg_off; i < seg_last; ++i) {
                 if (aborted) break;
                 const int slot = cslot;
                 const bool got = mbar_wait(full + slot, cphase, abort_flag, P.err, 2 + (i % DEC_NW == warp ? 1 : 0));
@@ -359,7 +363,7 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS) decode_splitkv_kernel(c
                     if (lane == 0) mbar_arrive(empty + slot);
                     continue;
                 }
-                const int tok0 = (seg_page_begin + (i - seg_off)) * DEC_PT;
+                const int tok0 = seg_tok + i * DEC_PT;
                 const uint32_t kb = ksm_u + slot * PAGE_BYTES, vb = vsm_u + slot * PAGE_BYTES;
 
                 // ---- S = Q K^T for 16 tokens (two 8-token tiles)
@@ -389,7 +393,7 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS) decode_splitkv_kernel(c
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
                         const int tok = tok0 + nt * 8 + cq + e;
-                        t[nt * 2 + e] = tok < seg_kv_len ? s[nt][e] * P.scale_log2 : -INFINITY;
+                        t[nt * 2 + e] = (unsigned)tok < (unsigned)seg_len ? s[nt][e] * P.scale_log2 : -INFINITY;
                     }
                 float tmax = fmaxf(fmaxf(t[0], t[1]), fmaxf(t[2], t[3]));
                 tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 1));
@@ -474,7 +478,7 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS) decode_splitkv_kernel(c
             if (tid == 0) {
                 DecodeWalk w1 = *walk_s;
                 DecodeSegment s1;
-                *have_seg = decode_next_segment(P.kv_len, P.B, P.Hkv, T, (int)gridDim.x, (int)blockIdx.x, w1, s1) ? 1 : 0;
+                *have_seg = decode_next_segment(P.end, P.B, P.Hkv, T, (int)gridDim.x, (int)blockIdx.x, w1, s1) ? 1 : 0;
                 *walk_s = w1;
                 *seg_s = s1;
             }
@@ -487,7 +491,7 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS) decode_splitkv_kernel(c
 struct CombineParams {
     const float* part_o;
     const float* part_ml;
-    const int* kv_len;   // [B]
+    const int* end;      // [B] as in DecodeParams
     int B, Hkv, g, D;
     int grid;            // CTAs of the split-KV launch whose records these are
     DecodeOutput res;
@@ -591,7 +595,7 @@ __global__ void decode_combine_kernel(const CombineParams P) {
     const int h = blockIdx.x, b = blockIdx.y;
     const int hk = h / P.g, rr = h % P.g;
     int first_slot, n_rec;
-    decode_head_records(P.kv_len, P.B, P.Hkv, P.grid, b, hk, red, first_slot, n_rec);
+    decode_head_records(P.end, P.B, P.Hkv, P.grid, b, hk, red, first_slot, n_rec);
     if (n_rec == 1) return;
     int dg;
     float M, L;
@@ -622,7 +626,7 @@ __global__ void decode_combine_exchange_kernel(const CombineExchangeParams P) {
         const int b = (int)(row / Hq), h = (int)(row % Hq);
         const int hk = h / P.C.g, rr = h % P.C.g;
         int first_slot, n_rec;
-        decode_head_records(P.C.kv_len, P.C.B, P.C.Hkv, P.C.grid, b, hk, red, first_slot, n_rec);
+        decode_head_records(P.C.end, P.C.B, P.C.Hkv, P.C.grid, b, hk, red, first_slot, n_rec);
         int dg;
         float M, L;
         float4 acc;
@@ -682,7 +686,7 @@ struct AppendParams {
     __nv_bfloat16* k_pages;
     __nv_bfloat16* v_pages;
     const int* page_table;
-    const int* len_before;  // [B]
+    const int* end_before;  // [B] rows of each sequence before this append, from the start of its first page
     int max_pages, Hkv, D, n, B;
 };
 
@@ -694,7 +698,7 @@ __global__ void kvcache_append_kernel(const AppendParams P) {
         const int t = (int)((i / P.D) % P.n);
         const int hk = (int)((i / ((long long)P.D * P.n)) % P.Hkv);
         const int b = (int)(i / ((long long)P.D * P.n * P.Hkv));
-        const int pos = P.len_before[b] + t;
+        const int pos = P.end_before[b] + t;
         const int page = P.page_table[(long long)b * P.max_pages + pos / DEC_PT];
         const long long dst = (((long long)page * P.Hkv + hk) * DEC_PT + pos % DEC_PT) * P.D + d;
         const long long ksrc = b * P.ks[0] + hk * P.ks[1] + t * P.ks[2] + d;
@@ -707,7 +711,7 @@ __global__ void kvcache_append_kernel(const AppendParams P) {
 }
 
 // Dense export: out [B][Hkv][len][D] (strided, f32 or bf16); rows past a sequence's length are zero.
-// `skip[b]` tokens at the front of sequence b have been evicted and are not exported.
+// The first `front[b]` rows of a sequence's first page have been evicted and are not exported.
 struct GatherParams {
     void* k_out;
     void* v_out;
@@ -716,7 +720,8 @@ struct GatherParams {
     const __nv_bfloat16* k_pages;
     const __nv_bfloat16* v_pages;
     const int* page_table;
-    const int* kv_len;  // [B]
+    const int* end;    // [B]
+    const int* front;  // [B]
     int max_pages, Hkv, D, len, B;
 };
 
@@ -729,9 +734,10 @@ __global__ void kvcache_gather_kernel(const GatherParams P) {
         const int hk = (int)((i / ((long long)P.D * P.len)) % P.Hkv);
         const int b = (int)(i / ((long long)P.D * P.len * P.Hkv));
         float kf = 0.0f, vf = 0.0f;
-        if (t < P.kv_len[b]) {
-            const int page = P.page_table[(long long)b * P.max_pages + t / DEC_PT];
-            const long long src = (((long long)page * P.Hkv + hk) * DEC_PT + t % DEC_PT) * P.D + d;
+        const int pos = P.front[b] + t;
+        if (pos < P.end[b]) {
+            const int page = P.page_table[(long long)b * P.max_pages + pos / DEC_PT];
+            const long long src = (((long long)page * P.Hkv + hk) * DEC_PT + pos % DEC_PT) * P.D + d;
             kf = __bfloat162float(P.k_pages[src]);
             vf = __bfloat162float(P.v_pages[src]);
         }

@@ -48,13 +48,14 @@ struct RopeParams {
     __nv_bfloat16* k_pages;
     __nv_bfloat16* v_pages;
     const int* page_table;
-    const int* len_before;  // [B] cache length of each sequence before this append
+    const int* end_before;  // [B] rows of each sequence before this append, from the start of its first page
+    const int* front;       // [B] evicted rows among them
     int max_pages, Hkv;
     // common
     const float* cos_t;
     const float* sin_t;
     int B, n, D;
-    int start_pos;  // table row of token 0; < 0: each sequence's len_before
+    int start_pos;  // table row of token 0; < 0: each sequence's length before this append
     int interleaved;
     int heads_per_thread;  // vector kernel: heads a thread walks with one set of cos / sin values
 };
@@ -69,8 +70,8 @@ __global__ void __launch_bounds__(256) rope_append_kernel(const RopeParams P) {
         const int t = (int)((idx / half) % P.n);
         const int h = (int)((idx / ((long long)half * P.n)) % heads);
         const int b = (int)(idx / ((long long)half * P.n * heads));
-        const int before = P.len_before ? P.len_before[b] : 0;
-        const int row = (P.start_pos >= 0 ? P.start_pos : before) + t;
+        const int before = P.end_before ? P.end_before[b] : 0;
+        const int row = (P.start_pos >= 0 ? P.start_pos : before - P.front[b]) + t;
         const float c = __ldg(P.cos_t + (long long)row * half + i);
         const float s = __ldg(P.sin_t + (long long)row * half + i);
         const int da = P.interleaved ? 2 * i : i;
@@ -184,8 +185,8 @@ __global__ void __launch_bounds__(256) rope_append_vec_kernel(const RopeParams P
         const unsigned t = (unsigned)(r % (unsigned)P.n);
         const unsigned bg = (unsigned)(r / (unsigned)P.n);
         const unsigned hg = bg % groups, b = bg / groups;
-        const int before = P.len_before ? P.len_before[b] : 0;
-        const int row = (P.start_pos >= 0 ? P.start_pos : before) + (int)t;
+        const int before = P.end_before ? P.end_before[b] : 0;
+        const int row = (P.start_pos >= 0 ? P.start_pos : before - P.front[b]) + (int)t;
         const int i0 = (int)ch * 8;
         float c[8], s[8];
         rope_load8(P.cos_t, 0, (long long)row * half + i0, c);

@@ -200,6 +200,11 @@ int32_t fusor_cuda_kvcache_rope_append(fusor_cuda_kvcache* cache, const fusor_cu
  * off the table row on the host; a drop that is not a multiple of the page size moves the kept rows with two kernel
  * launches (through a staging buffer the cache allocates on first use), whatever the length. */
 int32_t fusor_cuda_kvcache_truncate_front(fusor_cuda_kvcache* cache, int32_t b, int32_t keep);
+/* The same eviction without moving rows: whole pages go back to the pool, and a remainder of up to 15 evicted rows stays
+ * at the front of the sequence's first page, where every operation on the cache skips it (the raw pools show it).  The
+ * rows move only when an append would otherwise need a page that the sequence or the pool does not have, or at the next
+ * fusor_cuda_kvcache_truncate_front. */
+int32_t fusor_cuda_kvcache_drop_front(fusor_cuda_kvcache* cache, int32_t b, int32_t keep);
 /* KvCache::current_seq_len (kv_cache.rs:65-67) of sequence b. */
 int32_t fusor_cuda_kvcache_seq_len(fusor_cuda_kvcache* cache, int32_t b, int32_t* len);
 /* Installs a caller-built mapping (host arrays): page_table [B][max_pages_per_seq], kv_len [B]. Entries beyond

@@ -351,7 +351,7 @@ class KvCache {
             vv.data = (char*)vv.data + skip * vv.stride[2] * (v.dtype() == DType::F32 ? 4 : 2);
             vk.shape[2] = vv.shape[2] = (int64_t)max_len_;
         } else if (current_seq_len() + (size_t)n > max_len_) {
-            for (int64_t b = 0; b < s[0]; ++b) dev_->check(fusor_cuda_kvcache_truncate_front(cache_, (int32_t)b, (int32_t)(max_len_ - n)));
+            for (int64_t b = 0; b < s[0]; ++b) dev_->check(fusor_cuda_kvcache_drop_front(cache_, (int32_t)b, (int32_t)(max_len_ - n)));
         }
         dev_->check(fusor_cuda_kvcache_append(cache_, &vk, &vv));
         batch_ = s[0];
