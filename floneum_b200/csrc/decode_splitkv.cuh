@@ -164,12 +164,109 @@ struct DecodeSmem {
     }
 };
 
+// Q fragments of one (sequence, kv head): row r of the MMA tile is query head r of the group, rows >= g are zero.
+template <int D>
+__device__ __forceinline__ void decode_load_q(const DecodeParams& P, int b, int hk, int lane, uint32_t (&qa)[D / 16][2]) {
+    const int r = lane >> 2, cq = (lane & 3) * 2;
+#pragma unroll
+    for (int ks = 0; ks < D / 16; ++ks) {
+        qa[ks][0] = 0;
+        qa[ks][1] = 0;
+    }
+    if (r >= P.g) return;
+    const long long qoff = (long long)b * P.q_sb + (long long)(hk * P.g + r) * P.q_sh;
+#pragma unroll
+    for (int ks = 0; ks < D / 16; ++ks) {
+        const int d0 = ks * 16 + cq;
+        if (P.q_dtype == 1) {
+            const __nv_bfloat16* qp = reinterpret_cast<const __nv_bfloat16*>(P.q) + qoff;
+            qa[ks][0] = *reinterpret_cast<const uint32_t*>(qp + d0);
+            qa[ks][1] = *reinterpret_cast<const uint32_t*>(qp + d0 + 8);
+        } else {  // f32 or f16 queries are rounded to bf16, the type of the cached keys
+            qa[ks][0] = pack_bf16(ld_as_float(P.q, P.q_dtype, qoff + d0), ld_as_float(P.q, P.q_dtype, qoff + d0 + 1));
+            qa[ks][1] = pack_bf16(ld_as_float(P.q, P.q_dtype, qoff + d0 + 8), ld_as_float(P.q, P.q_dtype, qoff + d0 + 9));
+        }
+    }
+}
+
+// One page (16 tokens from tok0 on, of which 0 .. len - 1 exist) into a warp's running state: K tile at shared address kb, V at vb.
+template <int D>
+__device__ __forceinline__ void decode_page(uint32_t kb, uint32_t vb, const uint32_t (&qa)[D / 16][2], int tok0, int len, float scale_log2,
+                                            int lane, float& m_run, float& l_run, float (&o)[D / 8][4]) {
+    constexpr int HALF_BYTES = DEC_PT * 128;      // one 64-column half of a page tile
+    const int cq = (lane & 3) * 2;                // column pair inside an 8-wide tile
+    const int lm_j = lane >> 3, lm_r = lane & 7;  // ldmatrix lane geometry
+    // ---- S = Q K^T for 16 tokens (two 8-token tiles)
+    float s[2][4];
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt) s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.0f;
+#pragma unroll
+    for (int kp = 0; kp < D / 32; ++kp) {
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+            const int token = nt * 8 + lm_r;
+            const int cc = kp * 4 + lm_j;  // 16-byte chunk of the row, 0..D/8-1
+            const uint32_t addr =
+                kb + (cc >> 3) * HALF_BYTES + token * 128 + (((cc & 7) ^ (token & 7)) << 4);
+            uint32_t bfr[4];
+            ldmatrix_x4(bfr, addr);
+            const uint32_t a0[4] = {qa[2 * kp][0], 0u, qa[2 * kp][1], 0u};
+            const uint32_t a1[4] = {qa[2 * kp + 1][0], 0u, qa[2 * kp + 1][1], 0u};
+            mma_bf16_16816(s[nt], a0, bfr[0], bfr[1]);
+            mma_bf16_16816(s[nt], a1, bfr[2], bfr[3]);
+        }
+    }
+    // ---- online softmax on this thread's 4 scores of row r
+    float t[4];
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int tok = tok0 + nt * 8 + cq + e;
+            t[nt * 2 + e] = (unsigned)tok < (unsigned)len ? s[nt][e] * scale_log2 : -INFINITY;
+        }
+    float tmax = fmaxf(fmaxf(t[0], t[1]), fmaxf(t[2], t[3]));
+    tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 1));
+    tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 2));
+    const float m_new = fmaxf(m_run, tmax);
+    const float m_sub = (m_new == -INFINITY) ? 0.0f : m_new;
+    const float alpha = fast_exp2(m_run - m_sub);
+    m_run = m_new;
+    // P is handed to the tensor cores as bf16 hi + bf16 lo (two MMAs per tile): 8 significant bits
+    // alone put sequences of a few tokens above the 2e-3 tolerance, and the tensor pipe is idle here.
+    const float p0 = fast_exp2(t[0] - m_sub), p1 = fast_exp2(t[1] - m_sub);
+    const float p2 = fast_exp2(t[2] - m_sub), p3 = fast_exp2(t[3] - m_sub);
+    const __nv_bfloat162 h01 = __floats2bfloat162_rn(p0, p1), h23 = __floats2bfloat162_rn(p2, p3);
+    const __nv_bfloat162 l01 = __floats2bfloat162_rn(p0 - __low2float(h01), p1 - __high2float(h01));
+    const __nv_bfloat162 l23 = __floats2bfloat162_rn(p2 - __low2float(h23), p3 - __high2float(h23));
+    l_run = l_run * alpha + (p0 + p1) + (p2 + p3);
+    const uint32_t pa[4] = {*reinterpret_cast<const uint32_t*>(&h01), 0u, *reinterpret_cast<const uint32_t*>(&h23), 0u};
+    const uint32_t pl[4] = {*reinterpret_cast<const uint32_t*>(&l01), 0u, *reinterpret_cast<const uint32_t*>(&l23), 0u};
+#pragma unroll
+    for (int nd = 0; nd < D / 8; ++nd) {
+        o[nd][0] *= alpha;
+        o[nd][1] *= alpha;
+    }
+    // ---- O += P V
+#pragma unroll
+    for (int ndp = 0; ndp < D / 16; ++ndp) {
+        const int token = (lm_j & 1) * 8 + lm_r;
+        const int cc = ndp * 2 + (lm_j >> 1);
+        const uint32_t addr = vb + (cc >> 3) * HALF_BYTES + token * 128 + (((cc & 7) ^ (token & 7)) << 4);
+        uint32_t bfr[4];
+        ldmatrix_x4_trans(bfr, addr);
+        mma_bf16_16816(o[2 * ndp], pa, bfr[0], bfr[1]);
+        mma_bf16_16816(o[2 * ndp + 1], pa, bfr[2], bfr[3]);
+        mma_bf16_16816(o[2 * ndp], pl, bfr[0], bfr[1]);
+        mma_bf16_16816(o[2 * ndp + 1], pl, bfr[2], bfr[3]);
+    }
+}
+
 template <int D>
 __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS) decode_splitkv_kernel(const __grid_constant__ CUtensorMap tmK,
                                                                      const __grid_constant__ CUtensorMap tmV,
                                                                      const __grid_constant__ DecodeParams P) {
     constexpr int PAGE_BYTES = DecodeSmem<D>::PAGE_BYTES;
-    constexpr int HALF_BYTES = DEC_PT * 128;  // one 64-column half of a page tile
     extern __shared__ uint8_t dec_smem_raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dec_smem_raw) + 1023) & ~uintptr_t(1023));
     const int R = P.ring;
@@ -246,9 +343,7 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS) decode_splitkv_kernel(c
         decode_walk_init(W, T, (int)gridDim.x, (int)blockIdx.x, walk0[1], walk0[2]);
         DecodeSegment S;
         // ------------------------------------------------------------------ producer warp
-        // Lane 0 owns the ring bookkeeping; the 2*(D/64) TMA copies of a page (K and V, 64 columns each) are
-        // issued by as many lanes in one warp instruction.
-        constexpr int NOPS = 2 * (D / 64);
+        // Lane 0 owns the ring bookkeeping; lanes 0 and 1 issue the K and the V copy of a page.
         int slot = 0, phase = 0;  // ring position of the next page; `phase` flips each time the ring wraps
         bool wrapped = false;
         bool ok = true;
@@ -272,13 +367,12 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS) decode_splitkv_kernel(c
                         if (good) mbar_arrive_expect_tx(full + slot, 2 * PAGE_BYTES);
                     }
                     ok = __shfl_sync(0xffffffffu, good, 0) != 0;
-                    if (ok && lane < NOPS) {
-                        // lanes 0, 2 copy the K halves, lanes 1, 3 the V halves (the tensor map is named statically)
+                    if (ok && lane < 2) {
+                        // lane 0 copies the K tile, lane 1 the V tile, both 64-column halves in one instruction
                         const int row = (phys * P.Hkv + S.hk) * DEC_PT;
-                        const int hf = lane >> 1;
-                        const size_t off = (size_t)slot * PAGE_BYTES + hf * HALF_BYTES;
-                        if (lane & 1) tma_load_2d(vsm + off, &tmV, full + slot, hf * 64, row);
-                        else tma_load_2d(ksm + off, &tmK, full + slot, hf * 64, row);
+                        const size_t off = (size_t)slot * PAGE_BYTES;
+                        if (lane & 1) tma_load_3d(vsm + off, &tmV, full + slot, 0, row, 0);
+                        else tma_load_3d(ksm + off, &tmK, full + slot, 0, row, 0);
                     }
                     if (++slot == R) {
                         slot = 0;
@@ -292,11 +386,8 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS) decode_splitkv_kernel(c
         // ------------------------------------------------------------------ consumer warps
         const int r = lane >> 2;          // row of the 16-row MMA tile = query head within the group
         const int cq = (lane & 3) * 2;    // column pair inside an 8-wide tile
-        const bool row_valid = r < P.g;
         bool aborted = false;
         int cslot = 0, cphase = 0;  // ring position of the next page of the CTA's stream
-        // ldmatrix lane geometry
-        const int lm_j = lane >> 3, lm_r = lane & 7;
         const uint32_t ksm_u = smem_u32(ksm), vsm_u = smem_u32(vsm);
         constexpr int NC = DEC_NW * 32;   // consumer threads
         constexpr int DG = D / 4;         // float4 column groups of a row
@@ -316,28 +407,8 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS) decode_splitkv_kernel(c
             const int front = P.front[seg_s->b], seg_len = seg_s->kv_len - front;
             // token 0 of page i of the CTA's stream, counted from the first row that has not been evicted
             const int seg_tok = (seg_s->page_begin - seg_off) * DEC_PT - front;
-            // Q fragments: rows >= g are zero.
             uint32_t qa[D / 16][2];
-#pragma unroll
-            for (int ks = 0; ks < D / 16; ++ks) {
-                qa[ks][0] = 0;
-                qa[ks][1] = 0;
-            }
-            if (row_valid) {
-                const long long qoff = (long long)seg_s->b * P.q_sb + (long long)(seg_s->hk * P.g + r) * P.q_sh;
-#pragma unroll
-                for (int ks = 0; ks < D / 16; ++ks) {
-                    const int d0 = ks * 16 + cq;
-                    if (P.q_dtype == 1) {
-                        const __nv_bfloat16* qp = reinterpret_cast<const __nv_bfloat16*>(P.q) + qoff;
-                        qa[ks][0] = *reinterpret_cast<const uint32_t*>(qp + d0);
-                        qa[ks][1] = *reinterpret_cast<const uint32_t*>(qp + d0 + 8);
-                    } else {  // f32 or f16 queries are rounded to bf16, the type of the cached keys
-                        qa[ks][0] = pack_bf16(ld_as_float(P.q, P.q_dtype, qoff + d0), ld_as_float(P.q, P.q_dtype, qoff + d0 + 1));
-                        qa[ks][1] = pack_bf16(ld_as_float(P.q, P.q_dtype, qoff + d0 + 8), ld_as_float(P.q, P.q_dtype, qoff + d0 + 9));
-                    }
-                }
-            }
+            decode_load_q<D>(P, seg_s->b, seg_s->hk, lane, qa);
             float m_run = -INFINITY, l_run = 0.0f;
             float o[D / 8][4];
 #pragma unroll
@@ -365,71 +436,7 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS) decode_splitkv_kernel(c
                 }
                 const int tok0 = seg_tok + i * DEC_PT;
                 const uint32_t kb = ksm_u + slot * PAGE_BYTES, vb = vsm_u + slot * PAGE_BYTES;
-
-                // ---- S = Q K^T for 16 tokens (two 8-token tiles)
-                float s[2][4];
-#pragma unroll
-                for (int nt = 0; nt < 2; ++nt) s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.0f;
-#pragma unroll
-                for (int kp = 0; kp < D / 32; ++kp) {
-#pragma unroll
-                    for (int nt = 0; nt < 2; ++nt) {
-                        const int token = nt * 8 + lm_r;
-                        const int cc = kp * 4 + lm_j;  // 16-byte chunk of the row, 0..D/8-1
-                        const uint32_t addr =
-                            kb + (cc >> 3) * HALF_BYTES + token * 128 + (((cc & 7) ^ (token & 7)) << 4);
-                        uint32_t bfr[4];
-                        ldmatrix_x4(bfr, addr);
-                        const uint32_t a0[4] = {qa[2 * kp][0], 0u, qa[2 * kp][1], 0u};
-                        const uint32_t a1[4] = {qa[2 * kp + 1][0], 0u, qa[2 * kp + 1][1], 0u};
-                        mma_bf16_16816(s[nt], a0, bfr[0], bfr[1]);
-                        mma_bf16_16816(s[nt], a1, bfr[2], bfr[3]);
-                    }
-                }
-                // ---- online softmax on this thread's 4 scores of row r
-                float t[4];
-#pragma unroll
-                for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const int tok = tok0 + nt * 8 + cq + e;
-                        t[nt * 2 + e] = (unsigned)tok < (unsigned)seg_len ? s[nt][e] * P.scale_log2 : -INFINITY;
-                    }
-                float tmax = fmaxf(fmaxf(t[0], t[1]), fmaxf(t[2], t[3]));
-                tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 1));
-                tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 2));
-                const float m_new = fmaxf(m_run, tmax);
-                const float m_sub = (m_new == -INFINITY) ? 0.0f : m_new;
-                const float alpha = fast_exp2(m_run - m_sub);
-                m_run = m_new;
-                // P is handed to the tensor cores as bf16 hi + bf16 lo (two MMAs per tile): 8 significant bits
-                // alone put sequences of a few tokens above the 2e-3 tolerance, and the tensor pipe is idle here.
-                const float p0 = fast_exp2(t[0] - m_sub), p1 = fast_exp2(t[1] - m_sub);
-                const float p2 = fast_exp2(t[2] - m_sub), p3 = fast_exp2(t[3] - m_sub);
-                const __nv_bfloat162 h01 = __floats2bfloat162_rn(p0, p1), h23 = __floats2bfloat162_rn(p2, p3);
-                const __nv_bfloat162 l01 = __floats2bfloat162_rn(p0 - __low2float(h01), p1 - __high2float(h01));
-                const __nv_bfloat162 l23 = __floats2bfloat162_rn(p2 - __low2float(h23), p3 - __high2float(h23));
-                l_run = l_run * alpha + (p0 + p1) + (p2 + p3);
-                const uint32_t pa[4] = {*reinterpret_cast<const uint32_t*>(&h01), 0u, *reinterpret_cast<const uint32_t*>(&h23), 0u};
-                const uint32_t pl[4] = {*reinterpret_cast<const uint32_t*>(&l01), 0u, *reinterpret_cast<const uint32_t*>(&l23), 0u};
-#pragma unroll
-                for (int nd = 0; nd < D / 8; ++nd) {
-                    o[nd][0] *= alpha;
-                    o[nd][1] *= alpha;
-                }
-                // ---- O += P V
-#pragma unroll
-                for (int ndp = 0; ndp < D / 16; ++ndp) {
-                    const int token = (lm_j & 1) * 8 + lm_r;
-                    const int cc = ndp * 2 + (lm_j >> 1);
-                    const uint32_t addr = vb + (cc >> 3) * HALF_BYTES + token * 128 + (((cc & 7) ^ (token & 7)) << 4);
-                    uint32_t bfr[4];
-                    ldmatrix_x4_trans(bfr, addr);
-                    mma_bf16_16816(o[2 * ndp], pa, bfr[0], bfr[1]);
-                    mma_bf16_16816(o[2 * ndp + 1], pa, bfr[2], bfr[3]);
-                    mma_bf16_16816(o[2 * ndp], pl, bfr[0], bfr[1]);
-                    mma_bf16_16816(o[2 * ndp + 1], pl, bfr[2], bfr[3]);
-                }
+                decode_page<D>(kb, vb, qa, tok0, seg_len, P.scale_log2, lane, m_run, l_run, o);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(empty + slot);
             }
@@ -484,6 +491,159 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS) decode_splitkv_kernel(c
             }
             named_bar_sync(1, NC);
         }
+    }
+}
+
+// ---------------------------------------------------------------------------------- short sequences: a cluster per head
+// Decode over a few thousand tokens is bound by latencies, not by HBM: in the kernel above the deal, the second launch and
+// its reads of the records take three times as long as the pages.  Here a cluster of C CTAs takes one (sequence, kv
+// head), CTA r its r-th share of the pages, and the C states meet in shared memory over the cluster: one launch, no records.
+// Page i goes to warp i % DCL_NW, which copies it into one of its own slots, waits for it and uses it: eight warps fill their
+// slots at once (a single producer needs 0.36 us per page, two thirds of the time of a long share), and a refill needs no
+// hand-over.  Merge: the warps' states are merged per CTA, every CTA pushes the column groups a CTA is to finish into that
+// CTA's slots, and after one cluster barrier each CTA folds its own in rank order.
+// In graphs, pages cold, 32 query heads on 8 kv heads of 128: one sequence of 1411 tokens 13.6 -> 6.6 us, 6000 tokens 19.9 ->
+// 10.6 us, four of 4096 24.3 -> 15.5 us, sixteen of 2048 34.2 -> 25.5 us (5.4 TB/s).
+constexpr int DCL_NW = 8;
+constexpr int DCL_THREADS = DCL_NW * 32;
+constexpr int DCL_SLOTS = 3;                       // pages in flight per warp: 192 KB per SM at head_dim 128
+constexpr int DCL_MAX = 8;                         // most CTAs per cluster
+
+template <int D>
+struct DecodeClusterSmem {
+    static constexpr int PAGE_BYTES = DEC_PT * D * 2;
+    static constexpr int SLOT_F4 = DEC_GP * D / 4 + DCL_MAX;  // column groups pushed here by all CTAs (rounded up per source)
+    static constexpr size_t bytes = 1024 + (size_t)DCL_NW * DCL_SLOTS * 2 * PAGE_BYTES + (size_t)SLOT_F4 * 16 + DCL_NW * DEC_GP * 8 +
+                                    DCL_MAX * DEC_GP * 8 + DCL_NW * DCL_SLOTS * 8 + 64;
+};
+
+template <int D>
+__global__ void __launch_bounds__(DCL_THREADS, 1) decode_cluster_kernel(const __grid_constant__ CUtensorMap tmK,
+                                                                      const __grid_constant__ CUtensorMap tmV,
+                                                                      const __grid_constant__ DecodeParams P, const int C) {
+    using Smem = DecodeClusterSmem<D>;
+    constexpr int PAGE_BYTES = Smem::PAGE_BYTES, DG = D / 4, N_SLOTS = DCL_NW * DCL_SLOTS;
+    static_assert(2 * DCL_SLOTS * PAGE_BYTES >= DEC_GP * D * 4, "a warp's state fits its slots");
+    extern __shared__ uint8_t dec_smem_raw[];
+    uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dec_smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t* ring = base;                                                          // [warp][slot]{K page, V page}
+    float4* slots = reinterpret_cast<float4*>(ring + (size_t)N_SLOTS * 2 * PAGE_BYTES);  // [source CTA][column group of this CTA]
+    float* merge_ml = reinterpret_cast<float*>(slots + Smem::SLOT_F4);             // [NW][GP][2]
+    float2* slot_ml = reinterpret_cast<float2*>(merge_ml + DCL_NW * DEC_GP * 2);   // [source CTA][GP]
+    uint64_t* full = reinterpret_cast<uint64_t*>(slot_ml + DCL_MAX * DEC_GP);      // [warp][slot]
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(full + N_SLOTS);
+    // the warps' outputs [GP][D] at the end, each over its own slots
+    auto warp_out = [&](int w) { return reinterpret_cast<float*>(ring + (size_t)w * DCL_SLOTS * 2 * PAGE_BYTES); };
+
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int rank = C > 1 ? (int)cluster_cta_rank() : 0;
+    const int head = (int)blockIdx.x / C, b = head / P.Hkv, hk = head % P.Hkv;
+    const int end = P.end[b], front = P.front[b];
+    const int pages = (end + DEC_PT - 1) / DEC_PT;
+    const int p_begin = (int)((long long)pages * rank / C), p_end = (int)((long long)pages * (rank + 1) / C);
+    if (tid == 0) {
+        for (int i = 0; i < N_SLOTS; ++i) mbar_init(full + i, 1);
+        *abort_flag = 0;
+        mbar_fence_init();
+        tma_prefetch_desc(&tmK);
+        tma_prefetch_desc(&tmV);
+    }
+    __syncwarp();
+    if (C > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // waited for before the first push
+    __syncthreads();
+
+    {
+        const int n_mine = p_end - p_begin > warp ? (p_end - p_begin - warp + DCL_NW - 1) / DCL_NW : 0;  // pages of this warp
+        const int* pt = P.page_table + (long long)b * P.max_pages + p_begin + warp;
+        uint8_t* my_ring = ring + (size_t)warp * DCL_SLOTS * 2 * PAGE_BYTES;
+        uint64_t* my_full = full + warp * DCL_SLOTS;
+        int phys = 0;  // of this warp's pages 32 k + lane
+        auto copy = [&](int j) {  // the warp's page j into slot j % DCL_SLOTS
+            if ((j & 31) == 0) {
+                phys = j + lane < n_mine ? pt[(j + lane) * DCL_NW] : 0;
+                if (phys < 0 || phys >= P.num_pages) {  // record and read page 0 instead
+                    atomicExch(P.err, kErrBadPage);
+                    phys = 0;
+                }
+            }
+            const int row = (__shfl_sync(0xffffffffu, phys, j & 31) * P.Hkv + hk) * DEC_PT, slot = j % DCL_SLOTS;
+            if (lane == 0) {
+                mbar_arrive_expect_tx(my_full + slot, 2 * PAGE_BYTES);
+                tma_load_3d(my_ring + slot * 2 * PAGE_BYTES, &tmK, my_full + slot, 0, row, 0);
+                tma_load_3d(my_ring + slot * 2 * PAGE_BYTES + PAGE_BYTES, &tmV, my_full + slot, 0, row, 0);
+            }
+        };
+        for (int j = 0; j < min(n_mine, DCL_SLOTS); ++j) copy(j);
+        uint32_t qa[D / 16][2];
+        decode_load_q<D>(P, b, hk, lane, qa);
+        float m_run = -INFINITY, l_run = 0.0f;
+        float o[D / 8][4];
+#pragma unroll
+        for (int nd = 0; nd < D / 8; ++nd) o[nd][0] = o[nd][1] = o[nd][2] = o[nd][3] = 0.0f;
+        const uint32_t ring_u = smem_u32(my_ring);
+        for (int j = 0; j < n_mine; ++j) {
+            const int slot = j % DCL_SLOTS;
+            if (!__all_sync(0xffffffffu, mbar_wait(my_full + slot, (j / DCL_SLOTS) & 1, abort_flag, P.err, 4))) break;
+            const uint32_t kb = ring_u + slot * 2 * PAGE_BYTES;
+            decode_page<D>(kb, kb + PAGE_BYTES, qa, (p_begin + warp + j * DCL_NW) * DEC_PT - front, end - front, P.scale_log2, lane, m_run, l_run, o);
+            __syncwarp();  // every lane has read the slot
+            if (j + DCL_SLOTS < n_mine) copy(j + DCL_SLOTS);
+        }
+        l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
+        l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
+        const int r = lane >> 2, cq = (lane & 3) * 2;
+        float* mo = warp_out(warp) + r * D;
+#pragma unroll
+        for (int nd = 0; nd < D / 8; ++nd) *reinterpret_cast<float2*>(mo + nd * 8 + cq) = make_float2(o[nd][0], o[nd][1]);
+        if ((lane & 3) == 0) {
+            merge_ml[(warp * DEC_GP + r) * 2 + 0] = m_run;
+            merge_ml[(warp * DEC_GP + r) * 2 + 1] = l_run;
+        }
+    }
+    __syncthreads();
+    if (C > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // every CTA of the cluster has started
+    const int items = P.g * DG;           // column groups of the result
+    const int per = (items + C - 1) / C;  // CTA k finishes items [k per, (k + 1) per)
+    for (int item = tid; item < items; item += DCL_THREADS) {
+        const int rr = item / DG, dg = item - rr * DG;
+        float M = -INFINITY;
+#pragma unroll
+        for (int w = 0; w < DCL_NW; ++w) M = fmaxf(M, merge_ml[(w * DEC_GP + rr) * 2]);
+        float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        float sum = 0.0f;
+#pragma unroll
+        for (int w = 0; w < DCL_NW; ++w) {
+            const float mw = merge_ml[(w * DEC_GP + rr) * 2];
+            const float a = (mw == -INFINITY) ? 0.0f : fast_exp2(mw - M);
+            const float4 ow = *reinterpret_cast<const float4*>(warp_out(w) + rr * D + dg * 4);
+            acc.x += a * ow.x; acc.y += a * ow.y; acc.z += a * ow.z; acc.w += a * ow.w;
+            sum += a * merge_ml[(w * DEC_GP + rr) * 2 + 1];
+        }
+        if (C == 1) {
+            decode_emit(P.res, D, P.g, b, hk, rr, dg, M, sum, acc);
+        } else {
+            const int to = item / per;
+            st_cluster_f4(map_to_cta(slots + rank * per + (item - to * per), (uint32_t)to), acc);
+            if (dg < C) st_cluster_f2(map_to_cta(slot_ml + rank * DEC_GP + rr, (uint32_t)dg), make_float2(M, sum));
+        }
+    }
+    if (C == 1) return;
+    __syncwarp();
+    cluster_sync();  // everything pushed here has arrived
+    for (int item = rank * per + tid; item < min(items, (rank + 1) * per); item += DCL_THREADS) {
+        const int rr = item / DG, dg = item - rr * DG;
+        float M = -INFINITY;
+        for (int k = 0; k < C; ++k) M = fmaxf(M, slot_ml[k * DEC_GP + rr].x);
+        float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        float sum = 0.0f;
+        for (int k = 0; k < C; ++k) {
+            const float2 ml = slot_ml[k * DEC_GP + rr];
+            const float a = (ml.x == -INFINITY) ? 0.0f : fast_exp2(ml.x - M);
+            const float4 ow = slots[k * per + item - rank * per];
+            acc.x += a * ow.x; acc.y += a * ow.y; acc.z += a * ow.z; acc.w += a * ow.w;
+            sum += a * ml.y;
+        }
+        decode_emit(P.res, D, P.g, b, hk, rr, dg, M, sum, acc);
     }
 }
 

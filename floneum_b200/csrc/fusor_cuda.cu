@@ -309,6 +309,8 @@ extern "C" int32_t fusor_cuda_ctx_create(int32_t device, void* stream, fusor_cud
         {(const void*)oproj_split_kernel, (int)OPS_SMEM_BYTES, "oproj_split_kernel"},
         {(const void*)decode_splitkv_kernel<128>, 227 * 1024, "decode_splitkv_kernel<128>"},
         {(const void*)decode_splitkv_kernel<64>, 227 * 1024, "decode_splitkv_kernel<64>"},
+        {(const void*)decode_cluster_kernel<128>, (int)DecodeClusterSmem<128>::bytes, "decode_cluster_kernel<128>"},
+        {(const void*)decode_cluster_kernel<64>, (int)DecodeClusterSmem<64>::bytes, "decode_cluster_kernel<64>"},
         {(const void*)attn_mma16_kernel<96, false, false>, (int)am_smem_bytes<96>, "attn_mma16_kernel<96>"},
         {(const void*)attn_mma16_kernel<96, false, true>, (int)am_smem_bytes<96>, "attn_mma16_kernel<96>"},
         {(const void*)attn_mma16_kernel<96, true, false>, (int)am_smem_bytes<96>, "attn_mma16_kernel<96>"},
@@ -1073,13 +1075,14 @@ extern "C" int32_t fusor_cuda_kvcache_create(fusor_cuda_ctx* ctx, int32_t max_ba
     c->page_used.assign(num_pages, 0);
     c->free_list.resize(num_pages);
     for (int i = 0; i < num_pages; ++i) c->free_list[i] = num_pages - 1 - i;  // pop_back hands out page 0 first
-    // 2-D tensor maps over the pools: {D, num_pages*Hkv*16 rows}, box {64, 16}, 128-byte swizzle
+    // tensor maps over the pools, {64 columns, num_pages*Hkv*16 rows, D/64 halves}: one copy brings a whole (page, head) tile,
+    // half after half, 128-byte swizzle
     for (int which = 0; which < 2; ++which) {
-        cuuint64_t dims[2] = {(cuuint64_t)head_dim, (cuuint64_t)num_pages * num_kv_heads * DEC_PT};
-        cuuint64_t strides[1] = {(cuuint64_t)head_dim * 2};
-        cuuint32_t box[2] = {64, DEC_PT};
-        cuuint32_t estr[2] = {1, 1};
-        CUresult r = ctx->encode(which ? &c->tmV : &c->tmK, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
+        cuuint64_t dims[3] = {64, (cuuint64_t)num_pages * num_kv_heads * DEC_PT, (cuuint64_t)head_dim / 64};
+        cuuint64_t strides[2] = {(cuuint64_t)head_dim * 2, 128};
+        cuuint32_t box[3] = {64, DEC_PT, (cuuint32_t)head_dim / 64};
+        cuuint32_t estr[3] = {1, 1, 1};
+        CUresult r = ctx->encode(which ? &c->tmV : &c->tmK, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3,
                                  which ? (void*)c->v_pages : (void*)c->k_pages, dims, strides, box, estr,
                                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -1564,6 +1567,34 @@ static int32_t decode_impl(fusor_cuda_ctx* ctx, fusor_cuda_kvcache* c, const fus
     }
     DeviceGuard guard(ctx->device);
     TRY(kv_sync_tables(c));
+    DecodeParams P{};
+    P.q = q->data; P.q_dtype = q->dtype; P.q_sb = q->stride[0]; P.q_sh = q->stride[1];
+    P.page_table = c->d_page_table; P.max_pages = c->max_pages; P.num_pages = c->num_pages;
+    P.end = c->d_end; P.front = c->d_front; P.B = B;
+    P.part_o = c->part_o; P.part_ml = c->part_ml;
+    P.Hkv = c->Hkv; P.g = g; P.scale_log2 = scale * 1.4426950408889634f; P.err = ctx->d_err;
+    P.res.out = out; P.res.out_dtype = out_dtype; P.res.o_sb = o_sb; P.res.o_sh = o_sh; P.res.Hq = Hq; P.res.mode = mode;
+    // Short sequences: a cluster per (sequence, kv head), one launch.  C: the largest cluster of which all fit at once.
+    // Measured (8 KB pages, ns): the cluster takes 4600 + L max(126, 161 CTAs / 128) for a longest share of L pages, the even
+    // deal 13900 + 194 per page of an SM's share: 16 sequences of 256 .. 2048 tokens 25 against 27.5 us, of 512 .. 4096 tokens
+    // 46 against 37.  Below DCL_MAX pages most of a cluster has none: those calls keep the two launches that the test of the
+    // call pattern counts.
+    long long longest = 0;
+    for (int b = 0; b < B; ++b) longest = std::max<long long>(longest, pages_of(kv_end(c, b)));
+    const long long heads = (long long)B * c->Hkv, unit = 2ll * DEC_PT * c->D * 2;
+    if (mode != 2 && c->decode_ctas == 0 && heads <= ctx->num_sms && longest >= DCL_MAX) {
+        int i = 0;
+        while (i < 3 && heads <= ctx->clusters[i + 1]) ++i;
+        const int C = 1 << i;
+        const long long share = (longest + C - 1) / C, share_ns = share * std::max<long long>(126, 161 * heads * C / 128) * unit / 8192;
+        if (share_ns <= 9300 + total * 194 / ctx->num_sms * unit / 8192) {
+            cudaLaunchAttribute attr;
+            const cudaLaunchConfig_t cfg = cluster_config(ctx, (unsigned)(heads * C), (unsigned)C, DCL_THREADS,
+                                                          c->D == 128 ? DecodeClusterSmem<128>::bytes : DecodeClusterSmem<64>::bytes, &attr);
+            CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, c->D == 128 ? decode_cluster_kernel<128> : decode_cluster_kernel<64>, c->tmK, c->tmV, P, C));
+            return launch_check(ctx, "decode_cluster_kernel");
+        }
+    }
     // grid: whole multiples of the SM count while a CTA keeps a worthwhile share, never more CTAs than pages
     int per_sm = c->decode_ctas > 0 ? (c->decode_ctas + ctx->num_sms - 1) / ctx->num_sms
                                     : (int)std::max<long long>(1, std::min<long long>(DEC_CTAS, total / (kDecodeMinPagesPerCta * ctx->num_sms)));
@@ -1575,13 +1606,7 @@ static int32_t decode_impl(fusor_cuda_ctx* ctx, fusor_cuda_kvcache* c, const fus
     const int budget = (227 * 1024) / per_sm - 1024 - 1024 - DEC_NW * DEC_GP * (c->D + 2) * 4 - 1024;
     const int ring = std::max(2, std::min(24, budget / (2 * page_bytes + 16)));
     const size_t smem = c->D == 128 ? DecodeSmem<128>::bytes(ring) : DecodeSmem<64>::bytes(ring);
-    DecodeParams P{};
-    P.q = q->data; P.q_dtype = q->dtype; P.q_sb = q->stride[0]; P.q_sh = q->stride[1];
-    P.page_table = c->d_page_table; P.max_pages = c->max_pages; P.num_pages = c->num_pages;
-    P.end = c->d_end; P.front = c->d_front; P.B = B;
-    P.part_o = c->part_o; P.part_ml = c->part_ml;
-    P.Hkv = c->Hkv; P.g = g; P.scale_log2 = scale * 1.4426950408889634f; P.ring = ring; P.err = ctx->d_err;
-    P.res.out = out; P.res.out_dtype = out_dtype; P.res.o_sb = o_sb; P.res.o_sh = o_sh; P.res.Hq = Hq; P.res.mode = mode;
+    P.ring = ring;
     if (total > 0) {  // (every chunk empty: only the merge kernel runs and writes empty records)
         if (c->D == 128)
             decode_splitkv_kernel<128><<<grid, DEC_THREADS, smem, ctx->stream>>>(c->tmK, c->tmV, P);
@@ -1594,8 +1619,6 @@ static int32_t decode_impl(fusor_cuda_ctx* ctx, fusor_cuda_kvcache* c, const fus
     C.part_o = c->part_o; C.part_ml = c->part_ml; C.end = c->d_end;
     C.B = B; C.Hkv = c->Hkv; C.g = g; C.D = c->D; C.grid = grid; C.res = P.res;
     // record lanes per block: a kv head of a short sequence has one or two records, a 128 K-token sequence ~74
-    long long longest = 0;
-    for (int b = 0; b < B; ++b) longest = std::max<long long>(longest, pages_of(kv_end(c, b)));
     const long long per_head = longest * grid / std::max<long long>(1, total) + 2;
     const int lanes = per_head <= 4 ? 2 : per_head <= 32 ? 8 : DEC_CL;
     if (mode != 2) {
