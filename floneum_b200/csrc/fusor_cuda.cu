@@ -1242,6 +1242,23 @@ static int32_t rope_launch(fusor_cuda_ctx* ctx, const RopeParams& P) {
     if (vec && P.k_pages) vec = rope_vec_ok(P.k_new, P.k_dtype, P.ks) && rope_vec_ok(P.v_new, P.v_dtype, P.vs);
     const long long pairs = (long long)P.B * heads * P.n * (P.D / 2);
     RopeParams Q = P;
+    bool all16 = vec && P.q_dtype != FUSOR_CUDA_F32 && P.qo_dtype == P.q_dtype;
+    if (P.k_pages) all16 = all16 && P.k_dtype == P.q_dtype && P.v_dtype == P.q_dtype;
+    if (all16) {
+        // eight query heads a thread, halved while fewer than 1024 threads per SM would be left, down to two
+        const long long items = (long long)P.B * P.n * (P.D / 16);
+        auto threads_at = [&](int hpt) { return items * ((P.Hq + hpt - 1) / hpt + (P.k_pages ? (2 * P.Hkv + hpt - 1) / hpt : 0)); };
+        int hpt = 8;
+        while (hpt > 2 && threads_at(hpt) < 1024ll * ctx->num_sms) hpt /= 2;
+        Q.heads_per_thread = hpt;
+        const long long blocks = (threads_at(hpt) + 255) / 256;
+        if (blocks <= 0x7fffffffLL) {
+            auto run = [&](auto normal, auto interleaved) { (P.interleaved ? interleaved : normal)<<<(unsigned)blocks, 256, 0, ctx->stream>>>(Q); };
+            if (P.q_dtype == FUSOR_CUDA_F16) run(rope_append_16_kernel<false, true>, rope_append_16_kernel<true, true>);
+            else run(rope_append_16_kernel<false, false>, rope_append_16_kernel<true, false>);
+            return launch_check(ctx, "rope_append_16_kernel");
+        }
+    }
     long long threads = pairs;
     if (vec) {
         // enough (batch, token, chunk) items to fill the GPU twice over: let a thread walk several heads with its cos / sin
