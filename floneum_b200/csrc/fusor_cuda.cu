@@ -1013,7 +1013,8 @@ struct fusor_cuda_kvcache {
     std::vector<int> free_list;
     std::vector<char> page_used;
     int active_B = 0;
-    bool table_dirty = true;
+    bool table_dirty = true;  // the page table (and the lengths) on the device are behind
+    bool lens_dirty = false;  // only the lengths are
     CUtensorMap tmK, tmV;
     // split-KV decode: the kernel deals the pages out itself from d_end, the host only sizes the grid
     int max_grid = 0, max_slots = 0;
@@ -1123,7 +1124,7 @@ extern "C" int32_t fusor_cuda_kvcache_reset(fusor_cuda_kvcache* c) {
 // sequences (when a page was mapped or unmapped since the last upload)].  cudaMemcpyAsync from pageable memory returns
 // once the source has been staged, so the one staging vector can be refilled by the next call.
 static int32_t kv_upload_tables(fusor_cuda_kvcache* c, const int* before, int B) {
-    if (!before && !c->table_dirty) return FUSOR_CUDA_OK;
+    if (!before && !c->table_dirty && !c->lens_dirty) return FUSOR_CUDA_OK;
     fusor_cuda_ctx* ctx = c->ctx;
     const size_t mb = (size_t)c->max_batch;
     c->h_stage.resize(3 * mb + mb * c->max_pages);
@@ -1138,15 +1139,16 @@ static int32_t kv_upload_tables(fusor_cuda_kvcache* c, const int* before, int B)
         hi = 3 * mb + rows * c->max_pages;
     }
     CUDA_TRY(ctx, cudaMemcpyAsync(c->d_tables + lo, st + lo, (hi - lo) * 4, cudaMemcpyHostToDevice, ctx->stream));
-    c->table_dirty = false;
+    c->table_dirty = c->lens_dirty = false;
     return FUSOR_CUDA_OK;
 }
 static int32_t kv_sync_tables(fusor_cuda_kvcache* c) { return kv_upload_tables(c, nullptr, 0); }
 static int32_t kv_keep_rows(fusor_cuda_kvcache* c, int b, int keep);
 
 // Argument checks shared by the append entry points, then page allocation on the host: takes pages from the free list
-// for n more tokens per sequence, bumps the lengths and uploads the tables plus each sequence's previous length.
-static int32_t kv_reserve(fusor_cuda_kvcache* c, const fusor_cuda_tensor4* k_new, const fusor_cuda_tensor4* v_new) {
+// for n more tokens per sequence, bumps the lengths and brings them to the device: in `lens`, which the launch that follows
+// carries, or by uploading the tables plus each sequence's previous length.
+static int32_t kv_reserve(fusor_cuda_kvcache* c, const fusor_cuda_tensor4* k_new, const fusor_cuda_tensor4* v_new, KvLens* lens) {
     fusor_cuda_ctx* ctx = c->ctx;
     if (!dtype_ok(k_new->dtype) || !dtype_ok(v_new->dtype)) return fail(ctx, FUSOR_CUDA_INVALID_ARGUMENT, "unknown dtype");
     for (int i = 0; i < 4; ++i)
@@ -1190,25 +1192,36 @@ static int32_t kv_reserve(fusor_cuda_kvcache* c, const fusor_cuda_tensor4* k_new
     }
     c->active_B = B;
     if (need > 0) c->table_dirty = true;  // the page table travels only when a page was mapped
-    return kv_upload_tables(c, before.data(), B);
+    *lens = KvLens{};
+    lens->end_before = c->d_end_before; lens->front = c->d_front; lens->end_out = c->d_end; lens->front_out = c->d_front; lens->n = n;
+    if (c->table_dirty || B > KV_CARRY) return kv_upload_tables(c, before.data(), B);
+    lens->carried = B;
+    for (int b = 0; b < B; ++b) {
+        lens->end_v[b] = before[b];
+        lens->front_v[b] = c->h_front[b];
+    }
+    c->lens_dirty = false;
+    return FUSOR_CUDA_OK;
 }
 
 extern "C" int32_t fusor_cuda_kvcache_append(fusor_cuda_kvcache* c, const fusor_cuda_tensor4* k_new,
                                              const fusor_cuda_tensor4* v_new) {
     if (!c || !k_new || !v_new || !k_new->data || !v_new->data) return kv_fail(c, FUSOR_CUDA_INVALID_ARGUMENT, "null argument");
     fusor_cuda_ctx* ctx = c->ctx;
-    TRY(kv_reserve(c, k_new, v_new));
+    AppendParams P;
+    TRY(kv_reserve(c, k_new, v_new, &P.lens));
     DeviceGuard g(ctx->device);
     const int B = (int)k_new->shape[0], n = (int)k_new->shape[2];
-    AppendParams P;
     P.k_new = k_new->data; P.v_new = v_new->data; P.k_dtype = k_new->dtype; P.v_dtype = v_new->dtype;
     for (int i = 0; i < 3; ++i) { P.ks[i] = k_new->stride[i]; P.vs[i] = v_new->stride[i]; }
-    P.k_pages = c->k_pages; P.v_pages = c->v_pages; P.page_table = c->d_page_table; P.end_before = c->d_end_before;
+    P.k_pages = c->k_pages; P.v_pages = c->v_pages; P.page_table = c->d_page_table;
     P.max_pages = c->max_pages; P.Hkv = c->Hkv; P.D = c->D; P.n = n; P.B = B;
     const long long total = (long long)B * c->Hkv * n * c->D;
     const int blocks = (int)std::min<long long>((total + 255) / 256, (long long)ctx->num_sms * 8);
     kvcache_append_kernel<<<blocks, 256, 0, ctx->stream>>>(P);
-    return launch_check(ctx, "kvcache_append_kernel");
+    const int32_t rc = launch_check(ctx, "kvcache_append_kernel");
+    if (rc != FUSOR_CUDA_OK) c->lens_dirty = true;  // the lengths did not go with it
+    return rc;
 }
 
 // ------------------------------------------------------------------------------------------------ rotary embedding
@@ -1310,17 +1323,19 @@ extern "C" int32_t fusor_cuda_kvcache_rope_append(fusor_cuda_kvcache* c, const f
     }
     if (last > context_length)
         return fail(ctx, FUSOR_CUDA_INVALID_ARGUMENT, "positions up to %lld are outside the %d-row cos/sin tables", last, context_length);
-    TRY(kv_reserve(c, k_new, v_new));
-    DeviceGuard g(ctx->device);
     RopeParams P{};
+    TRY(kv_reserve(c, k_new, v_new, &P.lens));
+    DeviceGuard g(ctx->device);
     P.q = q->data; P.q_out = q_out->data; P.q_dtype = q->dtype; P.qo_dtype = q_out->dtype; P.Hq = (int)q->shape[1];
     for (int i = 0; i < 3; ++i) { P.qs[i] = q->stride[i]; P.qos[i] = q_out->stride[i]; P.ks[i] = k_new->stride[i]; P.vs[i] = v_new->stride[i]; }
     P.k_new = k_new->data; P.v_new = v_new->data; P.k_dtype = k_new->dtype; P.v_dtype = v_new->dtype;
-    P.k_pages = c->k_pages; P.v_pages = c->v_pages; P.page_table = c->d_page_table; P.end_before = c->d_end_before;
-    P.front = c->d_front; P.max_pages = c->max_pages; P.Hkv = c->Hkv;
+    P.k_pages = c->k_pages; P.v_pages = c->v_pages; P.page_table = c->d_page_table;
+    P.max_pages = c->max_pages; P.Hkv = c->Hkv;
     P.cos_t = cos_t; P.sin_t = sin_t; P.B = B; P.n = n; P.D = c->D; P.start_pos = start_pos < 0 ? -1 : start_pos;
     P.interleaved = interleaved ? 1 : 0;
-    return rope_launch(ctx, P);
+    const int32_t rc = rope_launch(ctx, P);
+    if (rc != FUSOR_CUDA_OK) c->lens_dirty = true;  // the lengths did not go with it
+    return rc;
 }
 
 extern "C" int32_t fusor_cuda_kvcache_seq_len(fusor_cuda_kvcache* c, int32_t b, int32_t* len) {
@@ -1503,11 +1518,14 @@ extern "C" int32_t fusor_cuda_kvcache_drop_front(fusor_cuda_kvcache* c, int32_t 
     DeviceGuard g(c->ctx->device);
     const int front = c->h_front[b] + drop;
     const int dp = keep == 0 ? pages_of(kv_end(c, b)) : front / DEC_PT;
-    kv_unmap_front(c, b, dp);
+    if (dp > 0) {
+        kv_unmap_front(c, b, dp);
+        c->table_dirty = true;
+    }
     c->h_kv_len[b] = keep;
     c->h_front[b] = keep == 0 ? 0 : front % DEC_PT;
-    c->table_dirty = true;
-    return kv_sync_tables(c);
+    c->lens_dirty = true;  // the append that follows, or the next use of the cache, brings the lengths to the device
+    return FUSOR_CUDA_OK;
 }
 
 // =============================================================================== decode

@@ -48,8 +48,7 @@ struct RopeParams {
     __nv_bfloat16* k_pages;
     __nv_bfloat16* v_pages;
     const int* page_table;
-    const int* end_before;  // [B] rows of each sequence before this append, from the start of its first page
-    const int* front;       // [B] evicted rows among them
+    KvLens lens;
     int max_pages, Hkv;
     // common
     const float* cos_t;
@@ -60,7 +59,8 @@ struct RopeParams {
     int heads_per_thread;  // vector kernels: heads (16-bit: query heads, or half as many kv heads) a thread walks with one set of cos / sin values
 };
 
-__global__ void __launch_bounds__(256) rope_append_kernel(const RopeParams P) {
+__global__ void __launch_bounds__(256) rope_append_kernel(const __grid_constant__ RopeParams P) {
+    if (P.k_pages) P.lens.publish();
     const int half = P.D >> 1;
     const int heads = P.Hq + (P.k_pages ? P.Hkv : 0);
     const long long total = (long long)P.B * heads * P.n * half;
@@ -70,8 +70,8 @@ __global__ void __launch_bounds__(256) rope_append_kernel(const RopeParams P) {
         const int t = (int)((idx / half) % P.n);
         const int h = (int)((idx / ((long long)half * P.n)) % heads);
         const int b = (int)(idx / ((long long)half * P.n * heads));
-        const int before = P.end_before ? P.end_before[b] : 0;
-        const int row = (P.start_pos >= 0 ? P.start_pos : before - P.front[b]) + t;
+        const int before = P.k_pages ? P.lens.before(b) : 0;
+        const int row = (P.start_pos >= 0 ? P.start_pos : before - P.lens.evicted(b)) + t;
         const float c = __ldg(P.cos_t + (long long)row * half + i);
         const float s = __ldg(P.sin_t + (long long)row * half + i);
         const int da = P.interleaved ? 2 * i : i;
@@ -171,7 +171,8 @@ __device__ __forceinline__ void rope_rotate8(float (&a)[8], float (&b)[8], const
 // A thread owns 8 pairs of one (batch, token) and walks `heads_per_thread` heads with them, so the cos / sin values it
 // loaded (64 bytes against 32 bytes of bf16 data per head) are reused instead of re-read from L2 for every head.
 template <bool INTERLEAVED>
-__global__ void __launch_bounds__(256) rope_append_vec_kernel(const RopeParams P) {
+__global__ void __launch_bounds__(256) rope_append_vec_kernel(const __grid_constant__ RopeParams P) {
+    if (P.k_pages) P.lens.publish();
     const int half = P.D >> 1;
     const unsigned chunks = (unsigned)half >> 3;  // 8 pairs per thread
     const unsigned heads = (unsigned)(P.Hq + (P.k_pages ? P.Hkv : 0));
@@ -185,8 +186,8 @@ __global__ void __launch_bounds__(256) rope_append_vec_kernel(const RopeParams P
         const unsigned t = (unsigned)(r % (unsigned)P.n);
         const unsigned bg = (unsigned)(r / (unsigned)P.n);
         const unsigned hg = bg % groups, b = bg / groups;
-        const int before = P.end_before ? P.end_before[b] : 0;
-        const int row = (P.start_pos >= 0 ? P.start_pos : before - P.front[b]) + (int)t;
+        const int before = P.k_pages ? P.lens.before(b) : 0;
+        const int row = (P.start_pos >= 0 ? P.start_pos : before - P.lens.evicted(b)) + (int)t;
         const int i0 = (int)ch * 8;
         float c[8], s[8];
         rope_load8(P.cos_t, 0, (long long)row * half + i0, c);
@@ -252,6 +253,7 @@ __device__ __forceinline__ void rope_unpack16(uint4 r, float (&f)[8]) {
 
 template <bool INTERLEAVED, bool F16>
 __global__ void __launch_bounds__(256) rope_append_16_kernel(const __grid_constant__ RopeParams P) {
+    if (P.k_pages) P.lens.publish();
     constexpr int U = 4, V = 2, DT = F16 ? 2 : 1;
     const int half = P.D >> 1;
     const unsigned chunks = (unsigned)half >> 3;  // 8 pairs per thread
@@ -266,8 +268,8 @@ __global__ void __launch_bounds__(256) rope_append_16_kernel(const __grid_consta
     const unsigned t = (unsigned)(r % (unsigned)P.n);
     const unsigned bg = (unsigned)(r / (unsigned)P.n);
     const unsigned grp = bg % groups, b = bg / groups;
-    const int before = P.end_before ? P.end_before[b] : 0;
-    const int row = (P.start_pos >= 0 ? P.start_pos : before - P.front[b]) + (int)t;
+    const int before = P.k_pages ? P.lens.before(b) : 0;
+    const int row = (P.start_pos >= 0 ? P.start_pos : before - P.lens.evicted(b)) + (int)t;
     const int i0 = (int)ch * 8;
     float c[8], s[8];
     const int offa = INTERLEAVED ? 2 * i0 : i0;

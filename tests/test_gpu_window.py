@@ -75,3 +75,26 @@ def test_a_pool_with_no_page_to_spare_takes_what_fits(device):
         assert [cache.seq_len(b) for b in range(2)] == [20, 0]
         got = cache.gather(2, 20)[0].as_slice()
         assert np.array_equal(got[0], k[0, :, 54:]) and not got[1].any()
+
+
+@pytest.mark.parametrize("B", [1, 32, 33])
+def test_lengths_reach_the_device_with_and_without_a_launch_that_carries_them(device, B):
+    """Appends that map no page bring the lengths in their launch (up to 32 sequences); a drop with no append after it, and the
+    plain append kernel, are seen by the next read all the same."""
+    fb = _fb()
+    rng = np.random.default_rng(B)
+    T = lambda a: fb.Tensor.from_slice(device, a.shape, np.ascontiguousarray(a))
+    k = O.bf16_round(rng.standard_normal((B, 1, 40, 64), dtype=np.float32))
+    q = O.bf16_round(rng.standard_normal((B, 2, 1, 64), dtype=np.float32))
+    cache = fb.PagedKvCache(device, B, 1, 64, 4 * B, 4)
+    lo = at = 0
+    for n, drop in ((20, 0), (3, 0), (1, 5), (0, 2), (9, 0), (2, 17), (1, 0), (0, 1)):
+        if n:
+            cache.append(T(k[:, :, at:at + n]), T(k[:, :, at:at + n]))
+            at += n
+        lo += drop
+        for b in range(B):
+            cache.drop_front(b, at - lo)
+        got = cache.decode(T(q), 0.125).as_slice()
+        assert_close(got, O.flash_attention(q, k[:, :, lo:at], k[:, :, lo:at], 0.125), what=f"{lo}..{at}")
+        assert np.array_equal(cache.gather(B, at - lo)[0].as_slice(), k[:, :, lo:at])
