@@ -52,11 +52,13 @@ class Device:
 
     def alloc(self, nbytes: int) -> int:
         p = ctypes.c_void_p()
-        _lib.check(self._L.fusor_cuda_buffer_alloc(self._h, nbytes, ctypes.byref(p)), self._h)
+        rc = self._L.fusor_cuda_buffer_alloc(self._h, nbytes, ctypes.byref(p))
+        if rc != _lib.OK:
+            _lib.check(rc, self._h)
         return p.value
 
     def free(self, ptr: int):
-        self._L.fusor_cuda_buffer_free(self._h, ctypes.c_void_p(ptr))
+        self._L.fusor_cuda_buffer_free(self._h, ptr)
 
     def close(self):
         if getattr(self, "_h", None):

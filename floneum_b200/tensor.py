@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import ctypes
 import enum
+import math
 from typing import Optional, Sequence, Tuple
 
 import numpy as np
@@ -52,22 +53,23 @@ class Tensor:
                  strides: Optional[Sequence[int]] = None, owner=None, owns: bool = False):
         self.device = device
         self.ptr = int(ptr)
-        self._shape = tuple(int(s) for s in shape)
+        self._shape = tuple(map(int, shape))
         self.dtype = dtype
         if strides is None:
-            strides, acc = [], 1
-            for s in reversed(self._shape):
-                strides.append(acc)
-                acc *= s
-            strides = tuple(reversed(strides))
-        self.strides = tuple(int(s) for s in strides)
+            strides, acc = [0] * len(self._shape), 1
+            for i in range(len(strides) - 1, -1, -1):
+                strides[i] = acc
+                acc *= self._shape[i]
+            self.strides = tuple(strides)
+        else:
+            self.strides = tuple(map(int, strides))
         self._owner = owner  # keeps a borrowed allocation (e.g. a torch tensor) alive
         self._owns = owns
 
     # ------------------------------------------------------------------ construction / readback
     @classmethod
     def empty(cls, device: Device, shape: Sequence[int], dtype: int = F32) -> "Tensor":
-        n = int(np.prod(shape)) if len(shape) else 1
+        n = math.prod(map(int, shape))
         ptr = device.alloc(max(n, 1) * _ITEMSIZE[dtype])
         return cls(device, ptr, shape, dtype, owns=True)
 
@@ -108,7 +110,7 @@ class Tensor:
         return True
 
     def numel(self) -> int:
-        return int(np.prod(self._shape)) if self._shape else 1
+        return math.prod(self._shape)
 
     def as_slice(self) -> np.ndarray:
         """Read back as a float32 numpy array indexable like the reference's TensorSlice."""
