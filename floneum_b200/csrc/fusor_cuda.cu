@@ -303,7 +303,8 @@ extern "C" int32_t fusor_cuda_ctx_create(int32_t device, void* stream, fusor_cud
     // opt in to large dynamic shared memory once per context (each call is checked by its own return value: a kernel
     // whose static shared memory pushes the sum over the limit must fail here, not at its first launch)
     struct { const void* fn; int bytes; const char* name; } opt_in[] = {
-        {(const void*)prefill_sm100_kernel, (int)PF_SMEM_BYTES, "prefill_sm100_kernel"},
+        {(const void*)prefill_sm100_kernel<false>, (int)PF_SMEM_BYTES, "prefill_sm100_kernel"},
+        {(const void*)prefill_sm100_kernel<true>, (int)PF_SMEM_BYTES, "prefill_sm100_kernel"},
         {(const void*)prefill2_sm100_kernel, (int)P2_SMEM_BYTES, "prefill2_sm100_kernel"},
         {(const void*)oproj_pair_kernel, (int)OP2_SMEM_BYTES, "oproj_pair_kernel"},
         {(const void*)oproj_split_kernel, (int)OPS_SMEM_BYTES, "oproj_split_kernel"},
@@ -693,10 +694,13 @@ static int32_t launch_prefill(fusor_cuda_ctx* ctx, const AttnShape& S, const fus
                               const fusor_cuda_tensor4* k, const fusor_cuda_tensor4* v, float scale, int32_t mask_kind,
                               const fusor_cuda_tensor4* out, int window = 0, const fusor_cuda_tensor2* key_mask = nullptr,
                               const fusor_cuda_tensor2* qk_mask = nullptr) {
-    // Two query tiles per CTA with 128-key blocks once a (batch, head) has 256 rows or more; the 64-key kernel with
-    // two CTAs per SM below that, and for calls with an additive [Sq, Skv] mask tensor (each softmax thread then reads a
-    // row of mask values per tile: the 64-key kernel has the registers for it).
-    const bool two_tiles = S.Sq >= P2_ROWS && qk_mask == nullptr;
+    // Two query tiles per CTA with 128-key blocks once the 256-row items outnumber the SMs; below that its CTAs each have one
+    // item and the call lasts as long as the longest, which 128-row tiles on twice the CTAs finish sooner (H32/8 causal, us,
+    // two tiles / one: S512 15.9 / 12.7, S1000 24.1 / 20.9, S1500 33.0 / 34.4 with 192 items; H8/8 S4096 67 / 60; B4 S300
+    // 21.3 / 18.1, where every second item is half empty).  Calls with an additive [Sq, Skv] mask tensor always take the 64-key
+    // kernel (each softmax thread reads a row of mask values per tile: it has the registers for that).
+    const long long items = (long long)((S.Sq + P2_ROWS - 1) / P2_ROWS) * S.Hq * S.B;
+    const bool two_tiles = S.Sq > P2_ROWS + P2_BM && items > ctx->num_sms && qk_mask == nullptr;
     const int kv_rows = two_tiles ? P2_BN : PF_BN;
     const bool in_f16 = q->dtype == FUSOR_CUDA_F16;  // f16 tensors need no copy of V: the weights are f16 against V itself
     CUtensorMap tmQ, tmK, tmV, tmV16, tmO;
@@ -754,7 +758,18 @@ static int32_t launch_prefill(fusor_cuda_ctx* ctx, const AttnShape& S, const fus
         prefill2_sm100_kernel<<<ctas, P2_THREADS, P2_SMEM_BYTES, ctx->stream>>>(tmQ, tmK, tmV, tmV16, tmO, P);
         return launch_check(ctx, "prefill2_sm100_kernel");
     }
-    prefill_sm100_kernel<<<(unsigned)grid, PF_THREADS, PF_SMEM_BYTES, ctx->stream>>>(tmQ, tmK, tmV, tmV16, tmO, P);
+    // Few tiles: parts of the keys on up to 8 CTAs each, two CTAs per SM.  The merge costs as much as four to six key tiles, so
+    // the longest row of tiles has to be 16 for two parts, and a part keeps more than 4.5.
+    const long long longest = (std::min(S.Skv, P.window > 0 ? P.window + PF_BM : S.Skv) + PF_BN - 1) / PF_BN;
+    int parts = 1;
+    while (parts < PF_MAX_SPLIT && grid * parts * 2 <= 2ll * ctx->num_sms && longest > (parts == 1 ? 15 : 9ll * parts)) parts *= 2;
+    if (parts > 1) {
+        cudaLaunchAttribute attr;
+        const cudaLaunchConfig_t cfg = cluster_config(ctx, (unsigned)(grid * parts), (unsigned)parts, PF_THREADS, PF_SMEM_BYTES, &attr);
+        CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, prefill_sm100_kernel<true>, tmQ, tmK, tmV, tmV16, tmO, P, parts));
+    } else {
+        prefill_sm100_kernel<false><<<(unsigned)grid, PF_THREADS, PF_SMEM_BYTES, ctx->stream>>>(tmQ, tmK, tmV, tmV16, tmO, P, 1);
+    }
     return launch_check(ctx, "prefill_sm100_kernel");
 }
 
@@ -2148,7 +2163,7 @@ extern "C" int32_t fusor_cuda_flash_attention_noalloc(void* stream, const fusor_
             cudaDriverEntryPointQueryResult qres;
             if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres) != cudaSuccess || !fn)
                 return fail(nullptr, FUSOR_CUDA_CUDA_ERROR, "cuTensorMapEncodeTiled is not available in this driver");
-            CUDA_TRY(nullptr, cudaFuncSetAttribute(prefill_sm100_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PF_SMEM_BYTES));
+            CUDA_TRY(nullptr, cudaFuncSetAttribute(prefill_sm100_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PF_SMEM_BYTES));
             nd.scratch = static_cast<unsigned char*>(p);
             nd.encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
             nd.num_sms = prop.multiProcessorCount;
@@ -2190,7 +2205,7 @@ extern "C" int32_t fusor_cuda_flash_attention_noalloc(void* stream, const fusor_
     P.n_q_tiles = (S.Sq + PF_BM - 1) / PF_BM;
     P.err = d_err;
     P.v_f16_overflow = d_overflow;
-    prefill_sm100_kernel<<<(unsigned)grid, PF_THREADS, PF_SMEM_BYTES, local.stream>>>(tmQ, tmK, tmV, tmV16, tmO, P);
+    prefill_sm100_kernel<false><<<(unsigned)grid, PF_THREADS, PF_SMEM_BYTES, local.stream>>>(tmQ, tmK, tmV, tmV16, tmO, P, 1);
     TRY(launch_check(&local, "prefill_sm100_kernel"));
     // Synchronous: wait for the result and report a device-side timeout of this call.
     int h_err = 0;

@@ -15,6 +15,14 @@
 // TMEM columns: S / P buffers from column 0 (PF_SBUF x PF_BN <= 128), O in [128,256).
 // All waits are bounded (ptx_sm100.cuh); on a timeout the CTA unwinds and frees its TMEM.
 //
+// SPLIT: a chain of tiles takes about a microsecond each whatever else runs, so a call with few query tiles (a follow-up on
+// a warm cache, few heads) leaves most SMs idle for the length of its longest row of tiles.  A cluster of up to 8 CTAs then
+// shares the key tiles of one query tile.  Each part ends with its own (m, l, O); the parts swap (m, l) through shared
+// memory over the cluster, scale their O to the common maximum and sum, and push the columns another CTA finishes into its
+// (idle) Q / K / V buffers; every CTA adds its 128 / C columns up in rank order and stores them.
+// H32/8, 64 new rows on 4000 cached keys 53 -> 24 us, 200 on 1000 20.0 -> 18.3 us; H8/1, 300 on 3000 44 -> 21 us; H8/8 S2048
+// causal 30 -> 23 us.  The merge costs 4 to 6 us, so 12 tiles are not split (14.8 us, 16.8 in two parts).
+//
 // Replaces the reference's fused kernel for Sq > 1
 // (fusor-ml/core/src/composite/flash_attention.rs:147-331: one subgroup per output row,
 // keys visited serially, mask read from a dense [Sq,Skv] tensor).
@@ -67,17 +75,20 @@ struct PrefillParams {
     long long qkmask_stride;   // elements between query rows
 };
 
-constexpr size_t PF_SMEM_BYTES = 1024 + (size_t)PF_Q_BYTES + 2 * PF_SBUF * (size_t)PF_KV_BYTES + 512 + 6 * 128 * 4;
+constexpr int PF_MAX_SPLIT = 8;
+constexpr size_t PF_SMEM_BYTES = 1024 + (size_t)PF_Q_BYTES + 2 * PF_SBUF * (size_t)PF_KV_BYTES + 512 + 2 * PF_MAX_SPLIT * 128 * 4;
+static_assert(PF_Q_BYTES + 2 * PF_SBUF * PF_KV_BYTES >= PF_BM * PF_D * 4, "the parts' columns fit the operand buffers");
 
 // P (the softmax weights handed to the second MMA) and V must have the same 16-bit type: kind::f16 rejects a
 // mixed f16 / bf16 operand pair.  bf16 weights (8 significant bits) put rows with few keys above the 2e-3
 // tolerance, so the host converts V to f16 once per call (cast_v_to_f16_kernel) and the kernel keeps P in f16
 // (11 bits).  When some |v| exceeds the f16 range the pre-pass raises a flag and every CTA falls back to bf16
 // P with the original bf16 V: the choice is a uniform runtime branch (descriptor bits and the tensor map).
+template <bool SPLIT>
 __global__ void __launch_bounds__(PF_THREADS, 2)
     prefill_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                          const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmV16,
-                         const __grid_constant__ CUtensorMap tmO, const PrefillParams P) {
+                         const __grid_constant__ CUtensorMap tmO, const PrefillParams P, const int parts) {
     extern __shared__ uint8_t pf_smem_raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(pf_smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* q_sm = base;
@@ -96,22 +107,29 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     float* xch = reinterpret_cast<float*>(bars + 32);  // [3][2 halves][128 rows]: partial maxima (2 buffers), row sums
+    float2* part_ml = reinterpret_cast<float2*>(xch);  // SPLIT: [part][128 rows] (m in log2 units, l)
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool use_f16 = P.in_f16 != 0 || (P.v_f16_overflow != nullptr && *P.v_f16_overflow == 0);
 
     // ---- which tile: heavy (late) query tiles first; consecutive CTAs share a kv head
     const int heads_total = P.Hq * P.B;
-    const int qt = P.n_q_tiles - 1 - (int)(blockIdx.x / heads_total);
-    const int hb = blockIdx.x % heads_total;
+    const int part = SPLIT ? (int)cluster_cta_rank() : 0, tile = SPLIT ? (int)blockIdx.x / parts : (int)blockIdx.x;
+    const int qt = P.n_q_tiles - 1 - tile / heads_total;
+    const int hb = tile % heads_total;
     const int h = hb % P.Hq, b = hb / P.Hq;
     const int hk = h / (P.Hq / P.Hkv);
     const int q0 = qt * PF_BM;
     const int offset = P.Skv - P.Sq;
     int n_kv = (P.Skv + PF_BN - 1) / PF_BN;  // becomes the number of key tiles this CTA visits, starting at tile j_begin
     if (P.causal) n_kv = min(n_kv, (q0 + PF_BM - 1 + offset) / PF_BN + 1);
-    const int j_begin = P.window > 0 ? max(0, q0 + offset - P.window + 1) / PF_BN : 0;
+    int j_begin = P.window > 0 ? max(0, q0 + offset - P.window + 1) / PF_BN : 0;
     n_kv -= j_begin;
+    if (SPLIT) {  // this part's tiles; none if there are fewer tiles than parts
+        const int first = n_kv * part / parts, last = n_kv * (part + 1) / parts;
+        j_begin += first;
+        n_kv = last - first;
+    }
 
     if (tid == 0) {
         mbar_init(q_full, 1);
@@ -139,6 +157,8 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    float m_ref = -INFINITY, l = 0.0f;  // of this thread's row (softmax warps)
+    bool ok = true;
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
@@ -182,7 +202,7 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
                 tc_commit(s_full + st);
                 tc_commit(k_empty + st);
             };
-            bool ok = mbar_wait(q_full, 0, abort_flag, P.err);
+            ok = mbar_wait(q_full, 0, abort_flag, P.err);
             for (int t = 0; t < PF_SBUF && t < n_kv && ok; ++t) {
                 ok = mbar_wait(k_full + t, 0, abort_flag, P.err);
                 if (ok) {
@@ -227,8 +247,6 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
         const float c = P.scale_log2;
         constexpr int OC = 128 / PF_TPR;  // output columns per thread
         const uint32_t o_tmem = tmem_base + lane_base + PF_COL_O + half * OC;
-        float m_ref = -INFINITY, l = 0.0f;
-        bool ok = true;
         for (int j = 0; j < n_kv && ok; ++j) {
             const int st = j % PF_SBUF;
             const uint32_t s_tmem = tmem_base + lane_base + PF_COL_S + st * PF_BN;
@@ -339,12 +357,12 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
             ok = mbar_wait(xch_bar + quad, n_kv & 1, abort_flag, P.err);
             if (ok) l += xch[(2 * 2 + (half ^ 1)) * 128 + row];
         }
-        if (ok) ok = mbar_wait(pv_done, (n_kv - 1) & 1, abort_flag, P.err);
+        if (ok && (!SPLIT || n_kv > 0)) ok = mbar_wait(pv_done, (n_kv - 1) & 1, abort_flag, P.err);
         // Epilogue: O / l goes through shared memory (the Q / K / V buffers are idle once the last MMA has
         // completed) in the 128-byte-swizzled layout of the output tensor map, then out with TMA stores:
         // full 128-byte lines instead of one 16-byte piece per row per instruction.  Rows past Sq are clipped.
         constexpr int BLK_BYTES = 128 * 128;  // one [128 rows][128 bytes] column block
-        if (ok) {
+        if (!SPLIT && ok) {
             tc_fence_after();
             const float inv_l = 1.0f / l;
 #pragma unroll
@@ -377,11 +395,90 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
         }
         // every softmax thread reaches this barrier, also after a timeout (then nothing is stored)
         const int any_failed = named_bar_or(1, 128 * PF_TPR, ok ? 0 : 1);
-        if (!any_failed && warp == 2 && lane == 0) {
+        ok = !any_failed;
+        if (!SPLIT && ok && warp == 2 && lane == 0) {
             const int n_blk = P.out_dtype == 0 ? 4 : 2, blk_cols = P.out_dtype == 0 ? 32 : 64;
             for (int kb = 0; kb < n_blk; ++kb) tma_store_4d(&tmO, base + kb * BLK_BYTES, kb * blk_cols, q0, h, b);
             tma_store_commit_and_wait_read();
         }
+    }
+    if (SPLIT) {
+        // ------------------------------------------------------------------ the parts of the tile meet
+        static_assert(PF_TPR == 1, "a softmax thread owns a row");
+        const int quad = warp & 3, row = quad * 32 + lane;
+        const uint32_t o_row = tmem_base + ((uint32_t)(quad * 32) << 16) + PF_COL_O;
+        __syncwarp();
+        cluster_sync();  // every part has started, and its operand buffers are idle: its last MMA and its loads are over
+        if (warp >= 2)
+            for (int k = 0; k < parts; ++k) st_cluster_f2(map_to_cta(part_ml + part * 128 + row, (uint32_t)k), make_float2(m_ref, l));
+        __syncwarp();
+        cluster_sync();
+        const int width = 128 / parts;  // columns a part finishes: 64, 32 or 16
+        float f = 0.0f;                 // what this part's O is multiplied by
+        if (warp >= 2) {
+            float M = -INFINITY, L = 0.0f;
+            for (int k = 0; k < parts; ++k) M = fmaxf(M, part_ml[k * 128 + row].x);
+            for (int k = 0; k < parts; ++k) {
+                const float2 ml = part_ml[k * 128 + row];
+                if (ml.x != -INFINITY) L += ml.y * fast_exp2(ml.x - M);
+            }
+            // (a row no part saw a key for: L = 0, and 0 * inf = NaN as without parts)
+            f = (m_ref == -INFINITY ? 0.0f : fast_exp2(m_ref - M)) * (1.0f / L);
+            tc_fence_after();
+        }
+        auto scaled = [&](int col, float (&v)[16]) {  // 16 columns of this part's O, scaled; 0 (or NaN) where it saw no tile
+            if (n_kv > 0) {
+                tmem_ld16(o_row + col, *reinterpret_cast<uint32_t(*)[16]>(&v[0]));
+                tc_wait_ld();
+            } else {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) v[i] = 0.0f;
+            }
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] *= f;
+        };
+        if (warp >= 2 && ok)
+            for (int col = 0; col < 128; col += 16) {
+                const int owner = col / width;
+                if (owner == part) continue;
+                float v[16];
+                scaled(col, v);
+                const uint32_t dst = map_to_cta(base, (uint32_t)owner) + (uint32_t)(((part * width + col - owner * width) / 4 * 128 + row) * 16);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) st_cluster_f4(dst + i * 128 * 16, make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]));
+            }
+        __syncwarp();
+        cluster_sync();  // all columns have arrived, and none is on its way to a CTA that leaves
+        if (warp >= 2 && ok)
+            for (int c0 = 0; c0 < width; c0 += 16) {
+                float own[16], sum[16];
+                scaled(part * width + c0, own);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) sum[i] = 0.0f;
+                for (int k = 0; k < parts; ++k) {
+                    const float4* src = reinterpret_cast<const float4*>(base) + (k * width + c0) / 4 * 128 + row;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float4 x = k == part ? make_float4(own[4 * i], own[4 * i + 1], own[4 * i + 2], own[4 * i + 3]) : src[i * 128];
+                        sum[4 * i] += x.x; sum[4 * i + 1] += x.y; sum[4 * i + 2] += x.z; sum[4 * i + 3] += x.w;
+                    }
+                }
+                if (q0 + row < P.Sq) {
+                    const long long at = (long long)b * P.os[0] + (long long)h * P.os[1] + (long long)(q0 + row) * P.os[2] + part * width + c0;
+                    if (P.out_dtype == 0) {
+                        float4* o = reinterpret_cast<float4*>(static_cast<float*>(P.out) + at);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) o[i] = make_float4(sum[4 * i], sum[4 * i + 1], sum[4 * i + 2], sum[4 * i + 3]);
+                    } else {
+                        uint4* o = reinterpret_cast<uint4*>(static_cast<uint16_t*>(P.out) + at);
+#pragma unroll
+                        for (int i = 0; i < 2; ++i)
+                            o[i] = make_uint4(pack_16(P.out_dtype, sum[8 * i], sum[8 * i + 1]), pack_16(P.out_dtype, sum[8 * i + 2], sum[8 * i + 3]),
+                                              pack_16(P.out_dtype, sum[8 * i + 4], sum[8 * i + 5]), pack_16(P.out_dtype, sum[8 * i + 6], sum[8 * i + 7]));
+                    }
+                }
+                __syncwarp();  // the next tcgen05.ld takes the whole warp
+            }
     }
     // ---- teardown: every role falls through to here, also after a timeout
     tc_fence_before();
