@@ -404,11 +404,12 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS) decode_splitkv_kernel(c
         while (*have_seg) {
             // what the page loop needs of the segment; the rest is read again from shared memory afterwards
             const int seg_off = seg_s->cta_page_off, seg_last = seg_off + seg_s->page_end - seg_s->page_begin;
-            const int front = P.front[seg_s->b], seg_len = seg_s->kv_len - front;
-            // token 0 of page i of the CTA's stream, counted from the first row that has not been evicted
-            const int seg_tok = (seg_s->page_begin - seg_off) * DEC_PT - front;
+            const int front = P.front[seg_s->b];  // first used after the loads of Q are on their way
             uint32_t qa[D / 16][2];
             decode_load_q<D>(P, seg_s->b, seg_s->hk, lane, qa);
+            const int seg_len = seg_s->kv_len - front;
+            // token 0 of page i of the CTA's stream, counted from the first row that has not been evicted
+            const int seg_tok = (seg_s->page_begin - seg_off) * DEC_PT - front;
             float m_run = -INFINITY, l_run = 0.0f;
             float o[D / 8][4];
 #pragma unroll
