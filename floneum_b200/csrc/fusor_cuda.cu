@@ -56,7 +56,9 @@ class BufferPool {
         if (take(size, out)) return cudaSuccess;
         auto waiting = freed_of_.find(size);
         if (waiting != freed_of_.end()) {
-            bool now = waiting->second >= std::max<size_t>(8, std::min<size_t>(256, (64u << 20) / size));
+            // 8 to 256, and before the buffers that wait fill half of what may be kept
+            const size_t enough = std::min(std::max<size_t>(8, std::min<size_t>(256, (64u << 20) / size)), std::max<size_t>(1, limit_ / 2 / size));
+            bool now = waiting->second >= enough;
             if (!now) {
                 now = cudaStreamQuery(stream) == cudaSuccess;
                 if (!now) cudaGetLastError();  // not ready
