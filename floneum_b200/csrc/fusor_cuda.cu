@@ -309,6 +309,7 @@ extern "C" int32_t fusor_cuda_ctx_create(int32_t device, void* stream, fusor_cud
         {(const void*)prefill_sm100_kernel<true>, (int)PF_SMEM_BYTES, "prefill_sm100_kernel"},
         {(const void*)prefill2_sm100_kernel, (int)P2_SMEM_BYTES, "prefill2_sm100_kernel"},
         {(const void*)oproj_pair_kernel, (int)OP2_SMEM_BYTES, "oproj_pair_kernel"},
+        {(const void*)oproj_single_kernel, (int)OP1_SMEM_BYTES, "oproj_single_kernel"},
         {(const void*)oproj_split_kernel, (int)OPS_SMEM_BYTES, "oproj_split_kernel"},
         {(const void*)decode_splitkv_kernel<128>, 227 * 1024, "decode_splitkv_kernel<128>"},
         {(const void*)decode_splitkv_kernel<64>, 227 * 1024, "decode_splitkv_kernel<64>"},
@@ -800,7 +801,7 @@ extern "C" int32_t fusor_cuda_flash_attention_general(fusor_cuda_ctx* ctx, const
 }
 
 // --------------------------------------------------------------------------- output projection
-// Which of the three kernels: by the number of output tiles, see oproj_sm100.cuh.
+// Which of the four kernels: by the number of output tiles, see oproj_sm100.cuh.
 static int32_t launch_out_proj(fusor_cuda_ctx* ctx, const fusor_cuda_tensor4* attn, const fusor_cuda_tensor4* w4,
                                const fusor_cuda_tensor4* out, OprojParams& P) {
     const long long rows = (long long)P.B * P.S, K = (long long)P.k_chunks * OP_BK;
@@ -829,7 +830,14 @@ static int32_t launch_out_proj(fusor_cuda_ctx* ctx, const fusor_cuda_tensor4* at
     TRY(make_tmap_bhsd(ctx, &tmO, out, 32, tmap_dtype(out->dtype)));
     P.n_tiles = (P.N + OP2_BN - 1) / OP2_BN;
     P.n_group = (int)std::max<long long>(1, std::min<long long>(P.n_tiles, (32ll << 20) / ((long long)OP2_BN * K * 2)));
-    const long long tiles = (m_tiles + 1) / 2 * P.n_tiles;
+    const long long tiles = (m_tiles + 1) / 2 * P.n_tiles, singles = m_tiles * P.n_tiles;
+    const long long pair_waves = (tiles + ctx->num_sms / 2 - 1) / (ctx->num_sms / 2), single_waves = (singles + ctx->num_sms - 1) / ctx->num_sms;
+    // a single tile takes 1.09 of a pair tile's time
+    if (singles <= 0x7fffffffLL && (109 * single_waves < 100 * pair_waves || (pair_waves == 1 && single_waves == 1 && P.k_chunks <= 24))) {
+        TRY(make_tmap_bhsd(ctx, &tmW, w4, OP1_BN));
+        oproj_single_kernel<<<(unsigned)std::min<long long>(singles, ctx->num_sms), OP_THREADS, OP1_SMEM_BYTES, ctx->stream>>>(tmA, tmW, tmO, P);
+        return launch_check(ctx, "oproj_single_kernel");
+    }
     if (tiles > 0x7fffffffLL) return fail(ctx, FUSOR_CUDA_UNSUPPORTED, "too many output tiles");
     const unsigned pairs = (unsigned)std::min<long long>(tiles, ctx->num_sms / 2);  // persistent: one CTA pair per two SMs
     oproj_pair_kernel<<<2 * pairs, OP_THREADS, OP2_SMEM_BYTES, ctx->stream>>>(tmA, tmW, tmO, P);

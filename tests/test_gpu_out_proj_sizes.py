@@ -1,4 +1,4 @@
-"""Output projection at the edges of its three kernels (a few rows, K split over a cluster, CTA pairs) against the oracle.
+"""Output projection at the edges of its four kernels (a few rows, K split over a cluster, CTA pairs, single CTAs) against the oracle.
 
 The products are exact in f32 and the sums have up to 4096 terms of N(0, 1) x N(0, 1 / K): another order of summation moves a
 result of size ~1 by a few units of sqrt(K) 2^-24 ~ 4e-6, well inside the bounds used here."""
@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("B,Hq,S,D,N", [
     (1, 1, 1, 64, 8), (1, 32, 1, 128, 4096), (8, 4, 1, 64, 136), (3, 5, 3, 64, 24), (2, 8, 8, 128, 264),  # a few rows: 1, 8, 9, 16; ragged N
     (1, 8, 17, 128, 40), (17, 2, 1, 64, 128), (1, 32, 129, 128, 384), (2, 16, 130, 128, 1032),            # K split 4, 1, 8, 2 ways
-    (1, 8, 700, 128, 3000), (3, 4, 1000, 128, 2056), (5, 2, 1100, 64, 512),                               # pairs: ragged, an odd number of row tiles
+    (1, 8, 700, 128, 3000), (3, 4, 1000, 128, 2056), (5, 2, 1100, 64, 512), (1, 16, 1300, 64, 2000),      # pairs, single CTAs: ragged, an odd number of row tiles
 ])
 @pytest.mark.parametrize("out_dtype", [0, 1])
 def test_out_proj_sizes(device, B, Hq, S, D, N, out_dtype):
