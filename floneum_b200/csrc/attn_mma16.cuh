@@ -75,10 +75,21 @@ constexpr int am_pitch = DP * 2 + 16;  // bytes of a row in shared memory
 template <int DP>
 constexpr size_t am_smem_bytes = (size_t)am_pitch<DP> * (AM_BM + 4 * AM_BN);
 
-// Online softmax of row r (0 or 1) of the thread's fragment: a row lives in the four threads of a quad.  m is the row maximum
-// in log2 units, l this thread's part of the row sum.  s becomes the weights.
+// s scale + mask with both steps rounded, as the composite computes it: next to a mask of -10000 the sum keeps 2^-11, and other
+// roundings would show there
+__device__ __forceinline__ void am_add_mask(float& s0, float& s1, float scale, float m0, float m1) {
+    const float2 x = fadd2(fmul2(make_float2(s0, s1), make_float2(scale, scale)), make_float2(m0, m1));
+    s0 = x.x;
+    s1 = x.y;
+}
+
+// Online softmax of row r (0 or 1) of the thread's fragment: a row lives in the four threads of a quad.  m is the row maximum,
+// l this thread's part of the row sum.  s becomes the weights.  Without a mask tensor s holds raw products, c = scale log2(e)
+// and m is in log2 units.  With one (ADD) s and m are in natural units and only differences are taken to log2: a finite mask
+// value down to the lowest float stays finite, so that a row in which every key carries it is the mean of V and not NaN.
 template <int BN, bool ADD>
-__device__ __forceinline__ void am_softmax_row(float (&s)[BN / 8][4], int r, float c, float2 c2, float& m, float& l, float& alpha) {
+__device__ __forceinline__ void am_softmax_row(float (&s)[BN / 8][4], int r, float c, float& m, float& l, float& alpha) {
+    constexpr float LOG2E = 1.4426950408889634f;
     float mx = fmaxf(s[0][2 * r], s[0][2 * r + 1]);
 #pragma unroll
     for (int nt = 1; nt < BN / 8; ++nt) mx = fmax3(mx, s[nt][2 * r], s[nt][2 * r + 1]);
@@ -87,13 +98,14 @@ __device__ __forceinline__ void am_softmax_row(float (&s)[BN / 8][4], int r, flo
     mx = fmaxf(m, ADD ? mx : mx * c);
     // a row whose keys so far are all masked keeps m = -inf: subtract 0, so that its weights are 0 and not NaN
     const float ms = mx == -INFINITY ? 0.0f : mx;
-    const float2 nm2 = make_float2(-ms, -ms);
-    alpha = fast_exp2(m - ms);
+    const float2 c2 = make_float2(c, c), e2 = make_float2(LOG2E, LOG2E), nm2 = make_float2(-ms, -ms);
+    alpha = fast_exp2(ADD ? (m - ms) * LOG2E : m - ms);
     m = mx;
     float2 sum = make_float2(0.0f, 0.0f);
 #pragma unroll
     for (int nt = 0; nt < BN / 8; ++nt) {
-        const float2 x = ffma2(make_float2(s[nt][2 * r], s[nt][2 * r + 1]), c2, nm2);
+        const float2 sv = make_float2(s[nt][2 * r], s[nt][2 * r + 1]);
+        const float2 x = ADD ? fmul2(fadd2(sv, nm2), e2) : ffma2(sv, c2, nm2);
         const float2 p = make_float2(fast_exp2(x.x), fast_exp2(x.y));
         s[nt][2 * r] = p.x;
         s[nt][2 * r + 1] = p.y;
@@ -143,7 +155,6 @@ __global__ void __launch_bounds__(AM_THREADS, DP <= 64 ? 3 : 2) attn_mma16_kerne
     extern __shared__ __align__(16) uint8_t am_smem[];
     constexpr int PITCH = am_pitch<DP>, CH = DP / 8;  // 16-byte chunks of a row
     constexpr int TERMS = F16 ? 2 : 3;
-    constexpr float LOG2E = 1.4426950408889634f;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t q_sm = smem_u32(am_smem);
     const uint32_t kv_sm = q_sm + AM_BM * PITCH;  // [2 buffers]{K, V}
@@ -180,7 +191,7 @@ __global__ void __launch_bounds__(AM_THREADS, DP <= 64 ? 3 : 2) attn_mma16_kerne
     const int r0 = q0 + warp * 16 + (lane >> 2);  // this thread's rows: r0 and r0 + 8
     const int cq = (lane & 3) * 2;                // column pair inside an 8-wide tile
     const int lm_j = lane >> 3, lm_r = lane & 7;
-    const float c = P.scale * LOG2E;  // scale > 0
+    const float c = P.scale * 1.4426950408889634f;  // scale > 0
     int first[2], last[2];            // keys each of the two rows may see
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
@@ -225,20 +236,16 @@ __global__ void __launch_bounds__(AM_THREADS, DP <= 64 ? 3 : 2) attn_mma16_kerne
                 mma_16816<F16>(s[nt], qa[2 * kp + 1], bf[2], bf[3]);
             }
         }
-        // ---- log2 units; additive masks, then the tile's edges (causal diagonal, window, past the last key)
-        float2 c2 = make_float2(c, c);
+        // ---- additive masks (natural units), then the tile's edges (causal diagonal, window, past the last key)
         if (ADD) {
 #pragma unroll
             for (int nt = 0; nt < AM_BN / 8; ++nt) {
                 const int kj = kt + nt * 8 + cq;
                 const float* k0 = mask0 + (long long)min(kj, P.Skv - 1) * P.ms[1];
                 const float* k1 = mask0 + (long long)min(kj + 1, P.Skv - 1) * P.ms[1];
-                s[nt][0] = fmaf(__ldg(k0), LOG2E, s[nt][0] * c);
-                s[nt][1] = fmaf(__ldg(k1), LOG2E, s[nt][1] * c);
-                s[nt][2] = fmaf(__ldg(k0 + mask_row8), LOG2E, s[nt][2] * c);
-                s[nt][3] = fmaf(__ldg(k1 + mask_row8), LOG2E, s[nt][3] * c);
+                am_add_mask(s[nt][0], s[nt][1], P.scale, __ldg(k0), __ldg(k1));
+                am_add_mask(s[nt][2], s[nt][3], P.scale, __ldg(k0 + mask_row8), __ldg(k1 + mask_row8));
             }
-            c2 = make_float2(1.0f, 1.0f);
         }
         if (kt + AM_BN > P.Skv || (causal && kt + AM_BN - 1 > q0 + warp * 16 + offset) ||
             (P.mask_kind == 4 && kt + P.window <= q0 + warp * 16 + 15 + offset)) {
@@ -250,10 +257,10 @@ __global__ void __launch_bounds__(AM_THREADS, DP <= 64 ? 3 : 2) attn_mma16_kerne
                     if (kj > last[e >> 1] || kj < first[e >> 1]) s[nt][e] = -INFINITY;
                 }
         }
-        // ---- online softmax; a row lives in the four threads of a quad.  m is the row maximum in log2 units.
+        // ---- online softmax
         float alpha[2];
 #pragma unroll
-        for (int r = 0; r < 2; ++r) am_softmax_row<AM_BN, ADD>(s, r, c, c2, m[r], l[r], alpha[r]);
+        for (int r = 0; r < 2; ++r) am_softmax_row<AM_BN, ADD>(s, r, c, m[r], l[r], alpha[r]);
         // ---- O = O alpha + P V.  The tile's product is summed by itself: the tensor core cuts off what lies below its running
         // sum, which over thousands of keys would show against f32 arithmetic; the sum over tiles is rounded properly.
         float t[DP / 8][4];

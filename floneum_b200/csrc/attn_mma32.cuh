@@ -39,7 +39,6 @@ __global__ void __launch_bounds__(AM_THREADS, DP <= 64 ? 2 : 1) attn_mma32_kerne
     extern __shared__ __align__(16) uint8_t am_smem[];
     constexpr int BN = a3_bn<DP>, PITCH = am_pitch<DP>, SP = a3_stage_pitch<DP>, CH = DP / 4;
     constexpr int QP = AM_BM * PITCH, KP = BN * PITCH;  // bytes of a plane
-    constexpr float LOG2E = 1.4426950408889634f;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t q_sm = smem_u32(am_smem), k_sm = q_sm + 3 * QP, v_sm = k_sm + 3 * KP, stage = v_sm + 3 * KP;
     uint8_t* stage_p = am_smem + (stage - q_sm);
@@ -98,7 +97,7 @@ __global__ void __launch_bounds__(AM_THREADS, DP <= 64 ? 2 : 1) attn_mma32_kerne
     const int r0 = q0 + warp * 16 + (lane >> 2);  // this thread's rows: r0 and r0 + 8
     const int cq = (lane & 3) * 2;                // column pair inside an 8-wide tile
     const int lm_j = lane >> 3, lm_r = lane & 7;
-    const float c = P.scale * LOG2E;  // scale > 0
+    const float c = P.scale * 1.4426950408889634f;  // scale > 0
     int first[2], last[2];            // keys each of the two rows may see
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
@@ -162,20 +161,16 @@ __global__ void __launch_bounds__(AM_THREADS, DP <= 64 ? 2 : 1) attn_mma32_kerne
                 mma_16816<false>(s[2 * np + 1], qa, kf[2], kf[3]);
             }
         }
-        // ---- log2 units; additive masks, then the tile's edges (causal diagonal, window, past the last key)
-        float2 c2 = make_float2(c, c);
+        // ---- additive masks (natural units), then the tile's edges (causal diagonal, window, past the last key)
         if (ADD) {
 #pragma unroll
             for (int nt = 0; nt < BN / 8; ++nt) {
                 const int kj = kt + nt * 8 + cq;
                 const float* k0 = mask0 + (long long)min(kj, P.Skv - 1) * P.ms[1];
                 const float* k1 = mask0 + (long long)min(kj + 1, P.Skv - 1) * P.ms[1];
-                s[nt][0] = fmaf(__ldg(k0), LOG2E, s[nt][0] * c);
-                s[nt][1] = fmaf(__ldg(k1), LOG2E, s[nt][1] * c);
-                s[nt][2] = fmaf(__ldg(k0 + mask_row8), LOG2E, s[nt][2] * c);
-                s[nt][3] = fmaf(__ldg(k1 + mask_row8), LOG2E, s[nt][3] * c);
+                am_add_mask(s[nt][0], s[nt][1], P.scale, __ldg(k0), __ldg(k1));
+                am_add_mask(s[nt][2], s[nt][3], P.scale, __ldg(k0 + mask_row8), __ldg(k1 + mask_row8));
             }
-            c2 = make_float2(1.0f, 1.0f);
         }
         if (kt + BN > P.Skv || (causal && kt + BN - 1 > q0 + warp * 16 + offset) ||
             (P.mask_kind == 4 && kt + P.window <= q0 + warp * 16 + 15 + offset)) {
@@ -189,7 +184,7 @@ __global__ void __launch_bounds__(AM_THREADS, DP <= 64 ? 2 : 1) attn_mma32_kerne
         }
         float alpha[2];
 #pragma unroll
-        for (int r = 0; r < 2; ++r) am_softmax_row<BN, ADD>(s, r, c, c2, m[r], l[r], alpha[r]);
+        for (int r = 0; r < 2; ++r) am_softmax_row<BN, ADD>(s, r, c, m[r], l[r], alpha[r]);
         // ---- O = O alpha + P V, the tile's product summed by itself (see attn_mma16.cuh)
         float t[DP / 8][4];
 #pragma unroll

@@ -2,7 +2,7 @@
 // operands with arbitrary batch/head/row strides, additive mask tensors (QKMask, BatchKeyMask)
 // or analytic causal / sliding-window masks.  It covers every call of the reference's
 // Tensor::flash_attention (fusor-ml/fusor/src/composite/flash_attention.rs:52-73) that the
-// tensor-core kernels do not take, and is the f32 path of the f32 CPU-reference configuration.
+// tensor-core kernels do not take (f32 and 16-bit tensors of head_dim up to 128 in aligned views: attn_mma32, attn_mma16).
 //
 // Bound by the FMA pipe.  One CTA = 8 RT query rows of one (batch, head), 128 threads as 8 row groups x 16 columns: a thread
 // owns RT rows (ty, ty + 8, ...) and, of each tile of 64 keys, the keys tx, tx + 16, tx + 32, tx + 48.  Q, K and V stand in
@@ -91,7 +91,6 @@ __global__ void __launch_bounds__(GEN_THREADS) general_attention_kernel(const __
     load(Qs, P.q, P.q_dtype, qbase, P.qs[2], BM, q0, P.Sq);
     load(Ks, P.k, P.k_dtype, kbase, P.ks[2], GEN_BN, k_begin, P.Skv);
 
-    const float c = P.scale * LOG2E;
     float m[RT], l[RT];
     float2 o[RT][2 * NC];
 #pragma unroll
@@ -129,7 +128,8 @@ __global__ void __launch_bounds__(GEN_THREADS) general_attention_kernel(const __
                 }
             }
         }
-        // ---- scale, mask, online softmax (log2 units)
+        // ---- scale, mask, online softmax, in natural units: only differences are taken to log2, so that finite mask values down
+        // to the lowest float stay finite
         const bool edge = kt + GEN_BN > P.Skv || (causal && kt + GEN_BN - 1 > q0 + offset) || (P.mask_kind == 4 && kt + P.window <= q0 + BM - 1 + offset);
         __syncwarp();  // the warp has read the P rows of the last tile
 #pragma unroll
@@ -139,10 +139,10 @@ __global__ void __launch_bounds__(GEN_THREADS) general_attention_kernel(const __
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int kj = kt + tx + 16 * j;
-                s[j] = (acc[r][j].x + acc[r][j].y) * c;
+                s[j] = __fmul_rn(acc[r][j].x + acc[r][j].y, P.scale);
                 if (P.mask != nullptr) {
                     const long long row = P.mask_kind == 1 ? min(qi, P.Sq - 1) : b;
-                    s[j] = fmaf(__ldg(P.mask + row * P.ms[0] + (long long)min(kj, P.Skv - 1) * P.ms[1]), LOG2E, s[j]);
+                    s[j] = __fadd_rn(s[j], __ldg(P.mask + row * P.ms[0] + (long long)min(kj, P.Skv - 1) * P.ms[1]));  // rounded as the composite does
                 }
                 if (edge && (kj >= P.Skv || (causal && kj > qi + offset) || (P.mask_kind == 4 && kj + P.window <= qi + offset))) s[j] = -INFINITY;
                 mx = fmaxf(mx, s[j]);
@@ -151,12 +151,12 @@ __global__ void __launch_bounds__(GEN_THREADS) general_attention_kernel(const __
             for (int i = 8; i > 0; i >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, i));
             // a row whose keys so far are all masked keeps m = -inf: subtract 0, so that its weights are 0 and not NaN
             const float ms = mx == -INFINITY ? 0.0f : mx;
-            const float alpha = fast_exp2(m[r] - ms);
+            const float alpha = fast_exp2((m[r] - ms) * LOG2E);
             m[r] = mx;
             float sum = 0.0f;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const float p = fast_exp2(s[j] - ms);
+                const float p = fast_exp2((s[j] - ms) * LOG2E);
                 sum += p;
                 Ps[(ty + 8 * r) * GEN_P_PITCH + tx + 16 * j] = p;
             }
