@@ -3,8 +3,10 @@
 //
 // The products q.k of 16-bit values are exact in f32, so S = Q K^T loses nothing on the tensor cores.  The softmax weights do
 // not fit 16 bits: they are handed over as a sum of 16-bit terms, two for f16 (22 significant bits) and three for bf16 (24),
-// each multiplied by the same V fragment.  The tcgen05 kernels keep one 11-bit term; callers of this path had f32 arithmetic
-// before (general_attention_kernel) and keep it.
+// each multiplied by the same V fragment.  f16 terms end at 2^-24, so f16 weights carry a factor of 2^14: what is lost of a weight
+// is below 2^-39 of the row's largest.  (Without the factor, 2^-25: with 2047 keys 17.4 nats below one other their sum was off by
+// 0.66 of itself, with it 3e-6.)  The tcgen05 kernels keep one 11-bit term; callers of this path had f32 arithmetic before
+// (general_attention_kernel) and keep it.
 //
 // One CTA = 64 query rows of one (batch, head), 4 warps x 16 rows; K and V tiles of 64 keys come by cp.async into two
 // buffers, rows padded by 16 bytes so that ldmatrix meets no bank conflict; Q stays in registers.  Three CTAs per SM
@@ -18,6 +20,7 @@
 namespace fusor {
 
 constexpr int AM_BM = 64, AM_BN = 64, AM_THREADS = 128;
+constexpr int AM_F16_SHIFT = 14;  // 2^14 times a weight of at most 1 is far from the largest f16
 
 struct AttnMmaParams {
     const void* q;
@@ -87,7 +90,8 @@ __device__ __forceinline__ void am_add_mask(float& s0, float& s1, float scale, f
 // l this thread's part of the row sum.  s becomes the weights.  Without a mask tensor s holds raw products, c = scale log2(e)
 // and m is in log2 units.  With one (ADD) s and m are in natural units and only differences are taken to log2: a finite mask
 // value down to the lowest float stays finite, so that a row in which every key carries it is the mean of V and not NaN.
-template <int BN, bool ADD>
+// SHIFT: weights and sums carry a factor of 2^SHIFT, which the division by l takes out again.
+template <int BN, bool ADD, int SHIFT>
 __device__ __forceinline__ void am_softmax_row(float (&s)[BN / 8][4], int r, float c, float& m, float& l, float& alpha) {
     constexpr float LOG2E = 1.4426950408889634f;
     float mx = fmaxf(s[0][2 * r], s[0][2 * r + 1]);
@@ -106,7 +110,8 @@ __device__ __forceinline__ void am_softmax_row(float (&s)[BN / 8][4], int r, flo
     for (int nt = 0; nt < BN / 8; ++nt) {
         const float2 sv = make_float2(s[nt][2 * r], s[nt][2 * r + 1]);
         const float2 x = ADD ? fmul2(fadd2(sv, nm2), e2) : ffma2(sv, c2, nm2);
-        const float2 p = make_float2(fast_exp2(x.x), fast_exp2(x.y));
+        float2 p = make_float2(fast_exp2(x.x), fast_exp2(x.y));
+        if (SHIFT) p = fmul2(p, make_float2(1 << SHIFT, 1 << SHIFT));  // (as a term of x it would cost the largest weights four bits)
         s[nt][2 * r] = p.x;
         s[nt][2 * r + 1] = p.y;
         sum = fadd2(sum, p);
@@ -260,7 +265,7 @@ __global__ void __launch_bounds__(AM_THREADS, DP <= 64 ? 3 : 2) attn_mma16_kerne
         // ---- online softmax
         float alpha[2];
 #pragma unroll
-        for (int r = 0; r < 2; ++r) am_softmax_row<AM_BN, ADD>(s, r, c, m[r], l[r], alpha[r]);
+        for (int r = 0; r < 2; ++r) am_softmax_row<AM_BN, ADD, F16 ? AM_F16_SHIFT : 0>(s, r, c, m[r], l[r], alpha[r]);
         // ---- O = O alpha + P V.  The tile's product is summed by itself: the tensor core cuts off what lies below its running
         // sum, which over thousands of keys would show against f32 arithmetic; the sum over tiles is rounded properly.
         float t[DP / 8][4];

@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(AM_THREADS, DP <= 64 ? 2 : 1) attn_mma32_kerne
         }
         float alpha[2];
 #pragma unroll
-        for (int r = 0; r < 2; ++r) am_softmax_row<BN, ADD>(s, r, c, m[r], l[r], alpha[r]);
+        for (int r = 0; r < 2; ++r) am_softmax_row<BN, ADD, 0>(s, r, c, m[r], l[r], alpha[r]);
         // ---- O = O alpha + P V, the tile's product summed by itself (see attn_mma16.cuh)
         float t[DP / 8][4];
 #pragma unroll

@@ -1,0 +1,51 @@
+"""Attention at f32 accuracy where few weights carry a row: small weights that add up, scores of tens of nats, values
+that have to be carried whole.  Against 64-bit softmax attention of the same inputs.
+
+With V = 1 on every key but the peak, V = 0 there, a row is the sum of its n small weights over their total: what it may be off
+by is the error of a score (the dot product's sums, below 6 x 2^-22 of a score of 20 nats, so 3e-5 of each weight) and, where
+weights are two f16 terms under a scale of 2^14, 2^-39 per weight."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _attention64(q, k, v, scale):
+    s = q.astype(np.float64) @ np.swapaxes(k.astype(np.float64), -1, -2) * scale
+    p = np.exp(s - s.max(-1, keepdims=True))
+    return p @ v.astype(np.float64) / p.sum(-1, keepdims=True)
+
+
+def _run(device, q, k, v, scale, dtype):
+    import floneum_b200 as fb
+    T = lambda a: fb.Tensor.from_slice(device, a.shape, np.ascontiguousarray(a), dtype)
+    return T(q).flash_attention(T(k), T(v), float(scale), None, 0).as_slice().astype(np.float64)
+
+
+@pytest.mark.parametrize("nats", [8, 14, 17.4, 20])
+@pytest.mark.parametrize("dtype,D,keys", [(2, 64, 2048), (2, 32, 300), (2, 96, 4099), (1, 64, 2048), (0, 64, 2048), (0, 128, 777), (0, 160, 777)])
+def test_small_weights_that_add_up(device, dtype, D, keys, nats):
+    rng = np.random.default_rng(int(10 * nats) + D)
+    rnd = {0: lambda a: a, 1: O.bf16_round, 2: lambda a: a.astype(np.float16).astype(np.float32)}[dtype]
+    u = rng.standard_normal(D).astype(np.float32)
+    u *= np.float32(np.sqrt(nats) * D ** 0.25 / np.linalg.norm(u))
+    q = rnd((u + 0.02 * rng.standard_normal((1, 1, 70, D))).astype(np.float32))
+    k = rnd((0.02 * rng.standard_normal((1, 1, keys, D)) + u * (np.arange(keys) == keys // 3)[:, None]).astype(np.float32))
+    v = np.ones((1, 1, keys, D), np.float32)
+    v[:, :, keys // 3] = 0.0
+    scale = np.float32(D ** -0.5)
+    want = _attention64(q, k, v, float(scale))
+    got = _run(device, q, k, v, scale, dtype)
+    bound = 3e-5 * want + (keys * 2.0 ** -39 if dtype == 2 else 0.0)
+    assert (np.abs(got - want) <= bound).all(), (np.abs(got - want) / want).max()
+
+
+def test_values_are_carried_whole(device):
+    """One key: the result is V itself, every bit of it."""
+    rng = np.random.default_rng(5)
+    for D in (64, 128):
+        q, k = (rng.standard_normal((1, 2, n, D), dtype=np.float32) for n in (3, 1))
+        v = (rng.standard_normal((1, 2, 1, D)) * 10.0 ** rng.integers(-20, 20, (1, 2, 1, D))).astype(np.float32)
+        assert np.array_equal(_run(device, q, k, v, 0.1, 0), np.broadcast_to(v, (1, 2, 3, D)).astype(np.float64))
