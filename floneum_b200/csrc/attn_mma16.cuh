@@ -60,17 +60,21 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4],
 // Two f32 -> packed 16-bit pair; x and y keep what the pair does not hold.
 template <bool F16>
 __device__ __forceinline__ uint32_t split_pair(float& x, float& y) {
+    uint32_t bits;
+    float2 f;
     if (F16) {
         const __half2 h = __floats2half2_rn(x, y);
-        const float2 f = __half22float2(h);
-        x -= f.x;
-        y -= f.y;
-        return *reinterpret_cast<const uint32_t*>(&h);
+        bits = *reinterpret_cast<const uint32_t*>(&h);
+        f = __half22float2(h);
+    } else {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+        bits = *reinterpret_cast<const uint32_t*>(&h);
+        f = make_float2(__uint_as_float(bits << 16), __uint_as_float(bits & 0xffff0000u));
     }
-    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
-    x -= __low2float(h);
-    y -= __high2float(h);
-    return *reinterpret_cast<const uint32_t*>(&h);
+    f = ffma2(f, make_float2(-1.0f, -1.0f), make_float2(x, y));
+    x = f.x;
+    y = f.y;
+    return bits;
 }
 
 template <int DP>
@@ -117,19 +121,6 @@ __device__ __forceinline__ void am_softmax_row(float (&s)[BN / 8][4], int r, flo
         sum = fadd2(sum, p);
     }
     l = l * alpha + (sum.x + sum.y);
-}
-
-// o = o alpha + t
-template <int DP>
-__device__ __forceinline__ void am_accumulate(float (&o)[DP / 8][4], const float (&t)[DP / 8][4], const float (&alpha)[2]) {
-#pragma unroll
-    for (int nd = 0; nd < DP / 8; ++nd)
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const float2 x = ffma2(make_float2(o[nd][2 * r], o[nd][2 * r + 1]), make_float2(alpha[r], alpha[r]), make_float2(t[nd][2 * r], t[nd][2 * r + 1]));
-            o[nd][2 * r] = x.x;
-            o[nd][2 * r + 1] = x.y;
-        }
 }
 
 // O / l (a fully masked row gives 0 * inf = NaN, as the reference)
@@ -228,17 +219,25 @@ __global__ void __launch_bounds__(AM_THREADS, DP <= 64 ? 3 : 2) attn_mma16_kerne
                 ldmatrix_x4(qa[ks], q_sm + (warp * 16 + (lm_j & 1) * 8 + lm_r) * PITCH + (ks * 2 + (lm_j >> 1)) * 16);
         }
         const uint32_t kb = kv_sm + buf * 2 * AM_BN * PITCH, vb = kb + AM_BN * PITCH;
-        // ---- S = Q K^T
+        // ---- S = Q K^T.  The tensor core cuts off what lies below its running sum, always towards zero, which shows against f32
+        // arithmetic: half as many steps per sum, and the two halves added with rounding.
         float s[AM_BN / 8][4];
 #pragma unroll
         for (int nt = 0; nt < AM_BN / 8; ++nt) {
+            float odd[4] = {};
             s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.0f;
 #pragma unroll
             for (int kp = 0; kp < DP / 32; ++kp) {
                 uint32_t bf[4];
                 ldmatrix_x4(bf, kb + (nt * 8 + lm_r) * PITCH + (kp * 4 + lm_j) * 16);
                 mma_16816<F16>(s[nt], qa[2 * kp], bf[0], bf[1]);
-                mma_16816<F16>(s[nt], qa[2 * kp + 1], bf[2], bf[3]);
+                mma_16816<F16>(odd, qa[2 * kp + 1], bf[2], bf[3]);
+            }
+#pragma unroll
+            for (int e = 0; e < 4; e += 2) {
+                const float2 x = fadd2(make_float2(s[nt][e], s[nt][e + 1]), make_float2(odd[e], odd[e + 1]));
+                s[nt][e] = x.x;
+                s[nt][e + 1] = x.y;
             }
         }
         // ---- additive masks (natural units), then the tile's edges (causal diagonal, window, past the last key)
@@ -248,8 +247,13 @@ __global__ void __launch_bounds__(AM_THREADS, DP <= 64 ? 3 : 2) attn_mma16_kerne
                 const int kj = kt + nt * 8 + cq;
                 const float* k0 = mask0 + (long long)min(kj, P.Skv - 1) * P.ms[1];
                 const float* k1 = mask0 + (long long)min(kj + 1, P.Skv - 1) * P.ms[1];
-                am_add_mask(s[nt][0], s[nt][1], P.scale, __ldg(k0), __ldg(k1));
-                am_add_mask(s[nt][2], s[nt][3], P.scale, __ldg(k0 + mask_row8), __ldg(k1 + mask_row8));
+                float m0 = __ldg(k0), m1 = __ldg(k1);
+                am_add_mask(s[nt][0], s[nt][1], P.scale, m0, m1);
+                if (mask_row8 != 0) {
+                    m0 = __ldg(k0 + mask_row8);
+                    m1 = __ldg(k1 + mask_row8);
+                }
+                am_add_mask(s[nt][2], s[nt][3], P.scale, m0, m1);
             }
         }
         if (kt + AM_BN > P.Skv || (causal && kt + AM_BN - 1 > q0 + warp * 16 + offset) ||
@@ -266,33 +270,44 @@ __global__ void __launch_bounds__(AM_THREADS, DP <= 64 ? 3 : 2) attn_mma16_kerne
         float alpha[2];
 #pragma unroll
         for (int r = 0; r < 2; ++r) am_softmax_row<AM_BN, ADD, F16 ? AM_F16_SHIFT : 0>(s, r, c, m[r], l[r], alpha[r]);
-        // ---- O = O alpha + P V.  The tile's product is summed by itself: the tensor core cuts off what lies below its running
-        // sum, which over thousands of keys would show against f32 arithmetic; the sum over tiles is rounded properly.
-        float t[DP / 8][4];
+        // ---- O = O alpha + P V.  For the same reason a tile's product is summed by itself, its first terms (four steps) apart from
+        // the small ones (cut far below), and the sum over tiles is rounded.
+        uint32_t pa[AM_BN / 16][TERMS][4];
 #pragma unroll
-        for (int i = 0; i < DP / 8; ++i) t[i][0] = t[i][1] = t[i][2] = t[i][3] = 0.0f;
-#pragma unroll
-        for (int kk = 0; kk < AM_BN / 16; ++kk) {
-            uint32_t pa[TERMS][4];
+        for (int kk = 0; kk < AM_BN / 16; ++kk)
 #pragma unroll
             for (int i = 0; i < TERMS; ++i) {
-                pa[i][0] = split_pair<F16>(s[2 * kk][0], s[2 * kk][1]);
-                pa[i][1] = split_pair<F16>(s[2 * kk][2], s[2 * kk][3]);
-                pa[i][2] = split_pair<F16>(s[2 * kk + 1][0], s[2 * kk + 1][1]);
-                pa[i][3] = split_pair<F16>(s[2 * kk + 1][2], s[2 * kk + 1][3]);
+                pa[kk][i][0] = split_pair<F16>(s[2 * kk][0], s[2 * kk][1]);
+                pa[kk][i][1] = split_pair<F16>(s[2 * kk][2], s[2 * kk][3]);
+                pa[kk][i][2] = split_pair<F16>(s[2 * kk + 1][0], s[2 * kk + 1][1]);
+                pa[kk][i][3] = split_pair<F16>(s[2 * kk + 1][2], s[2 * kk + 1][3]);
             }
 #pragma unroll
-            for (int nd = 0; nd < DP / 16; ++nd) {
+        for (int nd = 0; nd < DP / 16; ++nd) {
+            float big[2][4] = {}, small[2][4] = {};
+#pragma unroll
+            for (int kk = 0; kk < AM_BN / 16; ++kk) {
                 uint32_t bf[4];
                 ldmatrix_x4_trans(bf, vb + (kk * 16 + (lm_j & 1) * 8 + lm_r) * PITCH + (nd * 2 + (lm_j >> 1)) * 16);
+                mma_16816<F16>(big[0], pa[kk][0], bf[0], bf[1]);
+                mma_16816<F16>(big[1], pa[kk][0], bf[2], bf[3]);
 #pragma unroll
-                for (int i = TERMS - 1; i >= 0; --i) {
-                    mma_16816<F16>(t[2 * nd], pa[i], bf[0], bf[1]);
-                    mma_16816<F16>(t[2 * nd + 1], pa[i], bf[2], bf[3]);
+                for (int i = TERMS - 1; i > 0; --i) {
+                    mma_16816<F16>(small[0], pa[kk][i], bf[0], bf[1]);
+                    mma_16816<F16>(small[1], pa[kk][i], bf[2], bf[3]);
                 }
             }
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    float* x = &o[2 * nd + j][2 * r];
+                    const float2 y = fadd2(ffma2(make_float2(x[0], x[1]), make_float2(alpha[r], alpha[r]), make_float2(small[j][2 * r], small[j][2 * r + 1])),
+                                           make_float2(big[j][2 * r], big[j][2 * r + 1]));
+                    x[0] = y.x;
+                    x[1] = y.y;
+                }
         }
-        am_accumulate<DP>(o, t, alpha);
     }
     am_store<DP>(P, o, l, r0, cq, b, h);
 }

@@ -34,6 +34,19 @@ __device__ __forceinline__ void split3(float x, float y, uint32_t (&t)[3]) {
     }
 }
 
+// o = o alpha + t
+template <int DP>
+__device__ __forceinline__ void am_accumulate(float (&o)[DP / 8][4], const float (&t)[DP / 8][4], const float (&alpha)[2]) {
+#pragma unroll
+    for (int nd = 0; nd < DP / 8; ++nd)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const float2 x = ffma2(make_float2(o[nd][2 * r], o[nd][2 * r + 1]), make_float2(alpha[r], alpha[r]), make_float2(t[nd][2 * r], t[nd][2 * r + 1]));
+            o[nd][2 * r] = x.x;
+            o[nd][2 * r + 1] = x.y;
+        }
+}
+
 template <int DP, bool ADD>
 __global__ void __launch_bounds__(AM_THREADS, DP <= 64 ? 2 : 1) attn_mma32_kernel(const __grid_constant__ AttnMmaParams P) {
     extern __shared__ __align__(16) uint8_t am_smem[];

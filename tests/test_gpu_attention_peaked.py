@@ -49,3 +49,32 @@ def test_values_are_carried_whole(device):
         q, k = (rng.standard_normal((1, 2, n, D), dtype=np.float32) for n in (3, 1))
         v = (rng.standard_normal((1, 2, 1, D)) * 10.0 ** rng.integers(-20, 20, (1, 2, 1, D))).astype(np.float32)
         assert np.array_equal(_run(device, q, k, v, 0.1, 0), np.broadcast_to(v, (1, 2, 3, D)).astype(np.float64))
+
+
+@pytest.mark.parametrize("dtype", [0, 1, 2])
+@pytest.mark.parametrize("keys", [17, 100, 300])
+def test_error_of_short_rows(device, dtype, keys):
+    """Relative error of the whole result over ten inputs whose keys are 5 % outliers: no larger than that of f32 sums in order, which
+    is what served these tensors first.  The sums of such a row: D products (a rounding of half a unit each, the running sum
+    half the result on average), then one product per key: measured 0.7e-7 (bf16, 17 keys) to 4.6e-7 (f32, 300 keys)."""
+    D, errs, refs = 64, [], []
+    rnd = {0: lambda a: a, 1: O.bf16_round, 2: lambda a: a.astype(np.float16).astype(np.float32)}[dtype]
+    for seed in range(10):
+        rng = np.random.default_rng(seed)
+        q, k, v = (rnd((0.5 * rng.standard_normal((2, 4, keys, D))).astype(np.float32)) for _ in range(3))
+        k = rnd(np.where(rng.random((2, 4, keys, 1)) < 0.05, k * 8, k).astype(np.float32))
+        scale = np.float32(D ** -0.5)
+        want = _attention64(q, k, v, float(scale))
+        errs.append(np.linalg.norm(_run(device, q, k, v, scale, dtype) - want) / np.linalg.norm(want))
+        # the same in f32, every sum in order
+        s = np.zeros((2, 4, keys, keys), np.float32)
+        for d in range(D):
+            s += q[..., d, None] * k[..., None, :, d]
+        s *= scale
+        p = np.exp(s - s.max(-1, keepdims=True))
+        o, total = np.zeros(q.shape, np.float32), np.zeros(s.shape[:-1], np.float32)
+        for j in range(keys):
+            o += p[..., j, None] * v[..., j, None, :]
+            total += p[..., j]
+        refs.append(np.linalg.norm(o / total[..., None] - want) / np.linalg.norm(want))
+    assert np.mean(errs) <= 1.05 * np.mean(refs), (np.mean(errs), np.mean(refs))
