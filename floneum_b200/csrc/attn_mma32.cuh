@@ -1,8 +1,9 @@
 // Attention for f32 tensors on warp-level bf16 MMAs, with the accuracy of f32 arithmetic.
 //
-// An f32 value is the exact sum of three bf16 terms (8 significant bits each, cut off rather than rounded, so nothing
-// overflows).  A product of two such sums is taken as six of its nine partial products; the three left out lie below 2^-24 of
-// it, half a unit in the last place of an f32 product.  The warp MMA multiplies 1024 bf16 pairs per clock and SM, the FMA pipe
+// An f32 value is the exact sum of three bf16 terms, the first two rounded to nearest (cut off, every term has the value's sign,
+// and what the product leaves out reaches 2^-21 of it, always to one side).  A product of two such sums is taken as six of its
+// nine partial products; the three left out are at most 2^-23 of it and 2^-27 on average, to either side: the rounding of an f32
+// product is 2^-24 at most and 2^-26 on average.  The warp MMA multiplies 1024 bf16 pairs per clock and SM, the FMA pipe
 // 128 f32 pairs: with six products the MMA is ahead by a third, and it leaves the issue slots free for the softmax.
 //
 // One CTA = 64 query rows of one (batch, head), 4 warps x 16 rows.  K and V tiles arrive as f32 by cp.async in a staging
@@ -23,15 +24,17 @@ constexpr int a3_stage_pitch = DP * 4 + 16;  // bytes of an f32 row
 template <int DP>
 constexpr size_t a3_smem_bytes = (size_t)am_pitch<DP> * 3 * (AM_BM + 2 * a3_bn<DP>) + (size_t)a3_stage_pitch<DP> * 2 * a3_bn<DP>;
 
-// (x, y) -> three packed bf16 pairs whose sum is (x, y)
+// (x, y) -> three packed bf16 pairs whose sum is (x, y).  The first two are rounded to nearest, what is left then has at most 8
+// significant bits.
 __device__ __forceinline__ void split3(float x, float y, uint32_t (&t)[3]) {
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        const uint32_t a = __float_as_uint(x), b = __float_as_uint(y);
-        t[i] = __byte_perm(a, b, 0x7632);
-        x -= __uint_as_float(a & 0xffff0000u);
-        y -= __uint_as_float(b & 0xffff0000u);
+    for (int i = 0; i < 2; ++i) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+        t[i] = *reinterpret_cast<const uint32_t*>(&h);
+        x -= __uint_as_float(t[i] << 16);
+        y -= __uint_as_float(t[i] & 0xffff0000u);
     }
+    t[2] = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
 }
 
 // o = o alpha + t

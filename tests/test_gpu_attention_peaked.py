@@ -1,5 +1,5 @@
-"""Attention at f32 accuracy where few weights carry a row: small weights that add up, scores of tens of nats, values
-that have to be carried whole.  Against 64-bit softmax attention of the same inputs.
+"""Attention at f32 accuracy where few weights carry a row: small weights that add up, scores of tens of nats, operands whose
+mantissas are the worst for a split into 16-bit terms.  Against 64-bit softmax attention of the same inputs.
 
 With V = 1 on every key but the peak, V = 0 there, a row is the sum of its n small weights over their total: what it may be off
 by is the error of a score (the dot product's sums, below 6 x 2^-22 of a score of 20 nats, so 3e-5 of each weight) and, where
@@ -40,6 +40,28 @@ def test_small_weights_that_add_up(device, dtype, D, keys, nats):
     got = _run(device, q, k, v, scale, dtype)
     bound = 3e-5 * want + (keys * 2.0 ** -39 if dtype == 2 else 0.0)
     assert (np.abs(got - want) <= bound).all(), (np.abs(got - want) / want).max()
+
+
+@pytest.mark.parametrize("D", [8, 64, 128, 192])
+def test_products_of_f32_values_with_long_mantissas(device, D):
+    """Two keys whose scores of 40 nats are one product each, of a value whose low 16 mantissa bits are set and of the next value,
+    which has them clear.  In units of 2^-24 of 40 nats their difference may be off by 2 (what a split into three terms leaves out
+    of the product) and by 2 for the cut at the end of each of the two sums."""
+    rng = np.random.default_rng(D)
+    bits = np.concatenate([[0x3F80FFFF], 0x3F80FFFF | (rng.integers(0, 128, 63) << 16)]).astype(np.uint32)
+    x = bits.view(np.float32)
+    q = np.zeros((1, 64, 64, D), np.float32)
+    k = np.zeros((1, 64, 2, D), np.float32)
+    q[0, :, :, 3] = x
+    k[0, :, 0, 3], k[0, :, 1, 3] = x, (bits + 1).view(np.float32)
+    v = np.zeros((1, 64, 2, D), np.float32)
+    v[0, :, 0], v[0, :, 1] = 1.0, -1.0
+    top = x[None, :] * x[:, None].astype(np.float64)  # [head, row]
+    for scale in (40.0, 20.0, 10.0):
+        want = _attention64(q, k, v, scale)
+        got = _run(device, q, k, v, scale, 0)
+        slope = (1.0 - want ** 2) / 2.0  # of the result in the difference of the scores
+        assert (np.abs(got - want) <= slope * (scale * top[None, :, :, None]) * 6 * 2.0 ** -24 + 2.0 ** -22).all(), np.abs(got - want).max()
 
 
 def test_values_are_carried_whole(device):
