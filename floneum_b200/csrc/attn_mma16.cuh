@@ -123,24 +123,85 @@ __device__ __forceinline__ void am_softmax_row(float (&s)[BN / 8][4], int r, flo
     l = l * alpha + (sum.x + sum.y);
 }
 
+// Rows of a warp's 16 (bits of `rows`) again, in plain f32 arithmetic: a lane owns a key of every 32 and, for O, the columns
+// lane, lane + 32, ...  For operands that a sum of 16-bit terms does not stand for: next to an infinity its lower terms are zero or
+// NaN, and the largest floats round up to one.  All of these leave a NaN behind, which is what sends a row here; one that is NaN
+// by right (a NaN score) ends at its first tile.
+template <int DT>  // 0 = f32, 1 = bf16, 2 = f16
+__device__ __noinline__ void am_rows_f32(const AttnMmaParams& P, unsigned rows) {
+    // (its place is worked out again: as arguments these values cost the main loop of the callers 7 %)
+    const int hb = (int)(blockIdx.x % (unsigned)(P.Hq * P.B)), h = hb % P.Hq, b = hb / P.Hq;
+    const int row0 = (P.n_q_tiles - 1 - (int)(blockIdx.x / (unsigned)(P.Hq * P.B))) * AM_BM + (int)(threadIdx.x >> 5) * 16;
+    constexpr float LOG2E = 1.4426950408889634f;
+    const int lane = threadIdx.x & 31, hk = h / (P.Hq / P.Hkv), offset = P.Skv - P.Sq;
+    const bool causal = P.mask_kind == 3 || P.mask_kind == 4;
+    for (; rows != 0; rows &= rows - 1) {
+        const int qi = row0 + __ffs(rows) - 1;
+        const int last = causal ? min(P.Skv - 1, qi + offset) : P.Skv - 1, first = P.mask_kind == 4 ? max(0, qi + offset - P.window + 1) : 0;
+        const long long q_row = b * P.qs[0] + h * P.qs[1] + qi * P.qs[2], k_base = b * P.ks[0] + hk * P.ks[1], v_base = b * P.vs[0] + hk * P.vs[1];
+        float m = -INFINITY, l = 0.0f, acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        for (int kt = first; kt <= last && l == l; kt += 32) {
+            const int kj = kt + lane;
+            float s = -INFINITY;
+            if (kj <= last) {
+                float dot = 0.0f;
+                for (int d = 0; d < P.D; ++d) dot = fmaf(ld_as_float(P.q, DT, q_row + d), ld_as_float(P.k, DT, k_base + kj * P.ks[2] + d), dot);
+                s = __fmul_rn(dot, P.scale);
+                if (P.mask != nullptr) s = __fadd_rn(s, P.mask[(P.mask_kind == 1 ? qi : b) * P.ms[0] + kj * P.ms[1]]);
+            }
+            float mx = s;
+#pragma unroll
+            for (int i = 16; i > 0; i >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, i));
+            mx = fmaxf(m, mx);
+            const float ms = mx == -INFINITY ? 0.0f : mx, alpha = fast_exp2((m - ms) * LOG2E), p = fast_exp2((s - ms) * LOG2E);
+            m = mx;
+            float sum = p;
+#pragma unroll
+            for (int i = 16; i > 0; i >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, i);
+            l = l * alpha + sum;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[i] *= alpha;
+            for (int j = 0; j < min(32, last + 1 - kt); ++j) {
+                const float pj = __shfl_sync(0xffffffffu, p, j);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (lane + 32 * i < P.D) acc[i] = fmaf(pj, ld_as_float(P.v, DT, v_base + (kt + j) * P.vs[2] + lane + 32 * i), acc[i]);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (lane + 32 * i < P.D)
+                st_from_float(P.out, P.out_dtype, b * P.os[0] + h * P.os[1] + qi * P.os[2] + lane + 32 * i, l == l ? acc[i] * (1.0f / l) : l);
+    }
+}
+
 // O / l (a fully masked row gives 0 * inf = NaN, as the reference)
-template <int DP>
+template <int DP, int DT>
 __device__ __forceinline__ void am_store(const AttnMmaParams& P, const float (&o)[DP / 8][4], float (&l)[2], int r0, int cq, int b, int h) {
+    unsigned again = 0;  // rows of the warp that hold a NaN although some key has weight
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
         l[r] += __shfl_xor_sync(0xffffffffu, l[r], 1);
         l[r] += __shfl_xor_sync(0xffffffffu, l[r], 2);
         const int qi = r0 + r * 8;
-        if (qi >= P.Sq) continue;
         const float inv = 1.0f / l[r];
         const long long row = b * P.os[0] + h * P.os[1] + qi * P.os[2];
+        bool nan = false;
 #pragma unroll
         for (int nd = 0; nd < DP / 8; ++nd) {
             const int d = nd * 8 + cq;
-            if (d >= P.D) continue;
-            if (P.out_dtype == 0) *reinterpret_cast<float2*>(static_cast<float*>(P.out) + row + d) = make_float2(o[nd][2 * r] * inv, o[nd][2 * r + 1] * inv);
-            else *reinterpret_cast<uint32_t*>(static_cast<uint16_t*>(P.out) + row + d) = pack_16(P.out_dtype, o[nd][2 * r] * inv, o[nd][2 * r + 1] * inv);
+            if (d >= P.D || qi >= P.Sq) continue;
+            const float x = o[nd][2 * r] * inv, y = o[nd][2 * r + 1] * inv;
+            nan = nan || x != x || y != y;
+            if (P.out_dtype == 0) *reinterpret_cast<float2*>(static_cast<float*>(P.out) + row + d) = make_float2(x, y);
+            else *reinterpret_cast<uint32_t*>(static_cast<uint16_t*>(P.out) + row + d) = pack_16(P.out_dtype, x, y);
         }
+        unsigned lanes = __ballot_sync(0xffffffffu, nan && l[r] != 0.0f);
+        for (; lanes != 0; lanes &= lanes - 1) again |= 1u << (r * 8 + ((__ffs(lanes) - 1) >> 2));
+    }
+    if (again != 0) {
+        __syncwarp();  // the rows are stored again by other lanes
+        am_rows_f32<DT>(P, again);
     }
 }
 
@@ -309,7 +370,7 @@ __global__ void __launch_bounds__(AM_THREADS, DP <= 64 ? 3 : 2) attn_mma16_kerne
                 }
         }
     }
-    am_store<DP>(P, o, l, r0, cq, b, h);
+    am_store<DP, F16 ? 2 : 1>(P, o, l, r0, cq, b, h);
 }
 
 }  // namespace fusor

@@ -3,7 +3,7 @@
 // An f32 value is the exact sum of three bf16 terms, the first two rounded to nearest (cut off, every term has the value's sign,
 // and what the product leaves out reaches 2^-21 of it, always to one side).  A product of two such sums is taken as six of its
 // nine partial products; the three left out are at most 2^-23 of it and 2^-27 on average, to either side: the rounding of an f32
-// product is 2^-24 at most and 2^-26 on average.  The warp MMA multiplies 1024 bf16 pairs per clock and SM, the FMA pipe
+// product is 2^-24 at most and 2^-26 on average.  (Infinities and what rounds up to one: am_rows_f32.)  The warp MMA multiplies 1024 bf16 pairs per clock and SM, the FMA pipe
 // 128 f32 pairs: with six products the MMA is ahead by a third, and it leaves the issue slots free for the softmax.
 //
 // One CTA = 64 query rows of one (batch, head), 4 warps x 16 rows.  K and V tiles arrive as f32 by cp.async in a staging
@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(AM_THREADS, DP <= 64 ? 2 : 1) attn_mma32_kerne
             }
         am_accumulate<DP>(o, t, alpha);
     }
-    am_store<DP>(P, o, l, r0, cq, b, h);
+    am_store<DP, 0>(P, o, l, r0, cq, b, h);
 }
 
 }  // namespace fusor
