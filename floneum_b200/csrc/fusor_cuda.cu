@@ -305,9 +305,14 @@ extern "C" int32_t fusor_cuda_ctx_create(int32_t device, void* stream, fusor_cud
     // opt in to large dynamic shared memory once per context (each call is checked by its own return value: a kernel
     // whose static shared memory pushes the sum over the limit must fail here, not at its first launch)
     struct { const void* fn; int bytes; const char* name; } opt_in[] = {
-        {(const void*)prefill_sm100_kernel<false>, (int)PF_SMEM_BYTES, "prefill_sm100_kernel"},
-        {(const void*)prefill_sm100_kernel<true>, (int)PF_SMEM_BYTES, "prefill_sm100_kernel"},
-        {(const void*)prefill2_sm100_kernel, (int)P2_SMEM_BYTES, "prefill2_sm100_kernel"},
+        {(const void*)prefill_sm100_kernel<false, 0>, (int)PF_SMEM_BYTES, "prefill_sm100_kernel"},
+        {(const void*)prefill_sm100_kernel<false, 1>, (int)PF_SMEM_BYTES, "prefill_sm100_kernel"},
+        {(const void*)prefill_sm100_kernel<false, 2>, (int)PF_SMEM_BYTES, "prefill_sm100_kernel"},
+        {(const void*)prefill_sm100_kernel<true, 0>, (int)PF_SMEM_BYTES, "prefill_sm100_kernel"},
+        {(const void*)prefill_sm100_kernel<true, 1>, (int)PF_SMEM_BYTES, "prefill_sm100_kernel"},
+        {(const void*)prefill_sm100_kernel<true, 2>, (int)PF_SMEM_BYTES, "prefill_sm100_kernel"},
+        {(const void*)prefill2_sm100_kernel<false>, (int)P2_SMEM_BYTES, "prefill2_sm100_kernel"},
+        {(const void*)prefill2_sm100_kernel<true>, (int)P2_SMEM_BYTES, "prefill2_sm100_kernel"},
         {(const void*)oproj_pair_kernel, (int)OP2_SMEM_BYTES, "oproj_pair_kernel"},
         {(const void*)oproj_single_kernel, (int)OP1_SMEM_BYTES, "oproj_single_kernel"},
         {(const void*)oproj_split_kernel, (int)OPS_SMEM_BYTES, "oproj_split_kernel"},
@@ -758,7 +763,7 @@ static int32_t launch_prefill(fusor_cuda_ctx* ctx, const AttnShape& S, const fus
     if (grid > 0x7fffffffLL) return fail(ctx, FUSOR_CUDA_UNSUPPORTED, "grid too large");
     if (two_tiles) {
         const unsigned ctas = (unsigned)std::min<long long>(grid, ctx->num_sms);  // persistent: one CTA per SM
-        prefill2_sm100_kernel<<<ctas, P2_THREADS, P2_SMEM_BYTES, ctx->stream>>>(tmQ, tmK, tmV, tmV16, tmO, P);
+        (key_mask ? prefill2_sm100_kernel<true> : prefill2_sm100_kernel<false>)<<<ctas, P2_THREADS, P2_SMEM_BYTES, ctx->stream>>>(tmQ, tmK, tmV, tmV16, tmO, P);
         return launch_check(ctx, "prefill2_sm100_kernel");
     }
     // Few tiles: parts of the keys on up to 8 CTAs each, two CTAs per SM.  The merge costs as much as four to six key tiles, so
@@ -769,9 +774,10 @@ static int32_t launch_prefill(fusor_cuda_ctx* ctx, const AttnShape& S, const fus
     if (parts > 1) {
         cudaLaunchAttribute attr;
         const cudaLaunchConfig_t cfg = cluster_config(ctx, (unsigned)(grid * parts), (unsigned)parts, PF_THREADS, PF_SMEM_BYTES, &attr);
-        CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, prefill_sm100_kernel<true>, tmQ, tmK, tmV, tmV16, tmO, P, parts));
+        CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, qk_mask ? prefill_sm100_kernel<true, 2> : key_mask ? prefill_sm100_kernel<true, 1> : prefill_sm100_kernel<true, 0>, tmQ, tmK, tmV, tmV16, tmO, P, parts));
     } else {
-        prefill_sm100_kernel<false><<<(unsigned)grid, PF_THREADS, PF_SMEM_BYTES, ctx->stream>>>(tmQ, tmK, tmV, tmV16, tmO, P, 1);
+        (qk_mask ? prefill_sm100_kernel<false, 2> : key_mask ? prefill_sm100_kernel<false, 1> : prefill_sm100_kernel<false, 0>)
+            <<<(unsigned)grid, PF_THREADS, PF_SMEM_BYTES, ctx->stream>>>(tmQ, tmK, tmV, tmV16, tmO, P, 1);
     }
     return launch_check(ctx, "prefill_sm100_kernel");
 }
@@ -2173,7 +2179,7 @@ extern "C" int32_t fusor_cuda_flash_attention_noalloc(void* stream, const fusor_
             cudaDriverEntryPointQueryResult qres;
             if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres) != cudaSuccess || !fn)
                 return fail(nullptr, FUSOR_CUDA_CUDA_ERROR, "cuTensorMapEncodeTiled is not available in this driver");
-            CUDA_TRY(nullptr, cudaFuncSetAttribute(prefill_sm100_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PF_SMEM_BYTES));
+            CUDA_TRY(nullptr, cudaFuncSetAttribute(prefill_sm100_kernel<false, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PF_SMEM_BYTES));
             nd.scratch = static_cast<unsigned char*>(p);
             nd.encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
             nd.num_sms = prop.multiProcessorCount;
@@ -2215,7 +2221,7 @@ extern "C" int32_t fusor_cuda_flash_attention_noalloc(void* stream, const fusor_
     P.n_q_tiles = (S.Sq + PF_BM - 1) / PF_BM;
     P.err = d_err;
     P.v_f16_overflow = d_overflow;
-    prefill_sm100_kernel<false><<<(unsigned)grid, PF_THREADS, PF_SMEM_BYTES, local.stream>>>(tmQ, tmK, tmV, tmV16, tmO, P, 1);
+    prefill_sm100_kernel<false, 0><<<(unsigned)grid, PF_THREADS, PF_SMEM_BYTES, local.stream>>>(tmQ, tmK, tmV, tmV16, tmO, P, 1);
     TRY(launch_check(&local, "prefill_sm100_kernel"));
     // Synchronous: wait for the result and report a device-side timeout of this call.
     int h_err = 0;

@@ -63,6 +63,7 @@ __device__ __noinline__ void rescale_o_rows(uint32_t o_tmem, float alpha) {
     tc_wait_st();
 }
 
+template <bool KEY_MASK>
 __global__ void __launch_bounds__(P2_THREADS, 1)
     prefill2_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                           const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmV16,
@@ -321,12 +322,11 @@ __global__ void __launch_bounds__(P2_THREADS, 1)
                 for (int cc = 0; cc < 4; ++cc) tmem_ld32(s_tmem + cc * 32, *reinterpret_cast<uint32_t(*)[32]>(&s[cc * 32]));
                 tc_wait_ld();
                 const int k0 = (I.jb[t] + jj) * P2_BN;
-                if (P.kmask != nullptr) {
+                if (KEY_MASK) {
                     // additive key mask of this batch row: (s + mask / scale) * scale = s * scale + mask; every thread of the
                     // tile reads the same values (broadcast loads); keys past Skv are cut by the edge mask below
                     const float* mk = P.kmask + (long long)I.b * P.kmask_stride;
-#pragma unroll
-                    for (int i = 0; i < P2_BN; ++i) s[i] = fmaf(__ldg(mk + min(k0 + i, P.Skv - 1)), P.kmask_mul, s[i]);
+                    prefill_add_mask(P, mk, k0, s);
                 }
                 if (k0 + P2_BN - 1 > k_limit || k0 < k_first) {  // diagonal, ragged or window-edge block
 #pragma unroll
@@ -345,16 +345,20 @@ __global__ void __launch_bounds__(P2_THREADS, 1)
                     for (int a = 0; a < 8; ++a) mx[a] = fmax3(mx[a], s[i + 2 * a], s[i + 2 * a + 1]);
                 }
                 const float pmax = fmaxf(fmax3(mx[0], mx[1], mx[2]), fmaxf(fmax3(mx[3], mx[4], mx[5]), fmaxf(mx[6], mx[7])));
-                const float tmax = pmax * c;  // scale > 0
-                const float m_new = (tmax > m_ref + PF_RESCALE_THRESHOLD) ? tmax : m_ref;  // also taken on the first block
-                const float alpha = (m_new == -INFINITY) ? 1.0f : fast_exp2(m_ref - m_new);
+                const float tmax = KEY_MASK ? pmax : pmax * c;  // scale > 0; raw units with a mask, see prefill_mask
+                const float m_new = (tmax > m_ref + (KEY_MASK ? PF_RESCALE_THRESHOLD / c : PF_RESCALE_THRESHOLD)) ? tmax : m_ref;  // also taken on the first block
+                const float alpha = (m_new == -INFINITY) ? 1.0f : fast_exp2(KEY_MASK ? (m_ref - m_new) * c : m_ref - m_new);
                 m_ref = m_new;
                 // O must hold block jj-1 before it is rescaled and before any of P(jj) is handed over.  It does: S(jj) is
                 // ready, and the PV of block jj-1 was issued before S(jj) on the in-order pipe, so the commit that signalled
                 // S(jj) covers it.  No wait on pv_done here (it is observed once per item, before the epilogue; the barrier
                 // has then completed exactly the phases of all earlier blocks, so the parity of the last one is exact).
                 if (jj > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) rescale_o_rows(o_tmem, alpha);
-                const float m_sub = (m_ref == -INFINITY) ? 0.0f : m_ref;
+                float m_sub = (m_ref == -INFINITY) ? 0.0f : m_ref;
+                if (KEY_MASK) {
+                    prefill_subtract(m_sub, s);
+                    m_sub = 0.0f;
+                }
                 const float2 c2 = make_float2(c, c), nm2 = make_float2(-m_sub, -m_sub);
                 float2 ps0 = make_float2(0.0f, 0.0f), ps1 = make_float2(0.0f, 0.0f);
                 // Exponentials, software-pipelined by hand in groups of 4 elements: the warp issues in order and is alone on

@@ -79,12 +79,53 @@ constexpr int PF_MAX_SPLIT = 8;
 constexpr size_t PF_SMEM_BYTES = 1024 + (size_t)PF_Q_BYTES + 2 * PF_SBUF * (size_t)PF_KV_BYTES + 512 + 2 * PF_MAX_SPLIT * 128 * 4;
 static_assert(PF_Q_BYTES + 2 * PF_SBUF * PF_KV_BYTES >= PF_BM * PF_D * 4, "the parts' columns fit the operand buffers");
 
+// Two raw scores += mask / scale.  Finite values down to the lowest float would overflow to -inf in the quotient, and a row in which
+// every key carries them would be NaN instead of the mean of V: they are held at a floor, next to which a score disappears as it
+// does next to the value itself.  -inf stays -inf by the product with the least float, which is below 5e-7 for any other value.
+// For the same reason the maximum of a row stays in raw units where there is a mask tensor, and differences are taken before the
+// scaling: s scale - max of such values would not be 0 where s is the maximum.
+__device__ __forceinline__ void prefill_mask(const PrefillParams& P, float m0, float m1, float& s0, float& s1) {
+    const float2 m = make_float2(m0, m1), x = fmul2(m, make_float2(P.kmask_mul, P.kmask_mul));
+    const float2 s = fadd2(ffma2(m, make_float2(0x1p-149f, 0x1p-149f), make_float2(s0, s1)), make_float2(fmaxf(x.x, -1e38f), fmaxf(x.y, -1e38f)));
+    s0 = s.x;
+    s1 = s.y;
+}
+
+// s += the mask values `row` holds for the N keys from k0 on, four at a time where they are aligned and all there
+template <int N>
+__device__ __forceinline__ void prefill_add_mask(const PrefillParams& P, const float* row, int k0, float (&s)[N]) {
+    const float* m = row + k0;
+    if (k0 + N <= P.Skv && reinterpret_cast<uintptr_t>(m) % 16 == 0) {
+#pragma unroll
+        for (int i = 0; i < N; i += 4) {
+            const float4 x = __ldg(reinterpret_cast<const float4*>(m + i));
+            prefill_mask(P, x.x, x.y, s[i], s[i + 1]);
+            prefill_mask(P, x.z, x.w, s[i + 2], s[i + 3]);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; i += 2) prefill_mask(P, __ldg(row + min(k0 + i, P.Skv - 1)), __ldg(row + min(k0 + i + 1, P.Skv - 1)), s[i], s[i + 1]);
+    }
+}
+
+// s -= m
+template <int N>
+__device__ __forceinline__ void prefill_subtract(float m, float (&s)[N]) {
+#pragma unroll
+    for (int i = 0; i < N; i += 2) {
+        const float2 x = fadd2(make_float2(s[i], s[i + 1]), make_float2(-m, -m));
+        s[i] = x.x;
+        s[i + 1] = x.y;
+    }
+}
+
 // P (the softmax weights handed to the second MMA) and V must have the same 16-bit type: kind::f16 rejects a
 // mixed f16 / bf16 operand pair.  bf16 weights (8 significant bits) put rows with few keys above the 2e-3
 // tolerance, so the host converts V to f16 once per call (cast_v_to_f16_kernel) and the kernel keeps P in f16
 // (11 bits).  When some |v| exceeds the f16 range the pre-pass raises a flag and every CTA falls back to bf16
 // P with the original bf16 V: the choice is a uniform runtime branch (descriptor bits and the tensor map).
-template <bool SPLIT>
+// MASK: 0 = no mask tensor, 1 = a key mask, 2 = an [Sq, Skv] mask
+template <bool SPLIT, int MASK>
 __global__ void __launch_bounds__(PF_THREADS, 2)
     prefill_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                          const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmV16,
@@ -107,7 +148,7 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     float* xch = reinterpret_cast<float*>(bars + 32);  // [3][2 halves][128 rows]: partial maxima (2 buffers), row sums
-    float2* part_ml = reinterpret_cast<float2*>(xch);  // SPLIT: [part][128 rows] (m in log2 units, l)
+    float2* part_ml = reinterpret_cast<float2*>(xch);  // SPLIT: [part][128 rows] (m, l)
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool use_f16 = P.in_f16 != 0 || (P.v_f16_overflow != nullptr && *P.v_f16_overflow == 0);
@@ -158,6 +199,7 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     float m_ref = -INFINITY, l = 0.0f;  // of this thread's row (softmax warps)
+    const float m_unit = MASK ? P.scale_log2 : 1.0f;  // m_ref times this is in log2 units
     bool ok = true;
 
     if (warp == 0) {
@@ -245,6 +287,7 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
         const int k_limit = P.causal ? min(P.Skv - 1, qi + offset) : P.Skv - 1;  // last key this row may see
         const int k_first = P.window > 0 ? qi + offset - P.window + 1 : 0;      // first key this row may see
         const float c = P.scale_log2;
+        const float thr = MASK ? PF_RESCALE_THRESHOLD / c : PF_RESCALE_THRESHOLD;
         constexpr int OC = 128 / PF_TPR;  // output columns per thread
         const uint32_t o_tmem = tmem_base + lane_base + PF_COL_O + half * OC;
         for (int j = 0; j < n_kv && ok; ++j) {
@@ -259,19 +302,17 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
                 tmem_ld32(s_tmem + half * PF_CPT + cc * 32, *reinterpret_cast<uint32_t(*)[32]>(&s[cc * 32]));
             tc_wait_ld();
             const int k0 = (j_begin + j) * PF_BN + half * PF_CPT;
-            if (P.kmask != nullptr) {
+            if (MASK == 1) {
                 // additive key mask of this batch row: (s + mask / scale) * scale = s * scale + mask; every thread of the
                 // CTA reads the same values (broadcast loads); keys past Skv are cut by the edge mask below
                 const float* mk = P.kmask + (long long)b * P.kmask_stride;
-#pragma unroll
-                for (int i = 0; i < PF_CPT; ++i) s[i] = fmaf(__ldg(mk + min(k0 + i, P.Skv - 1)), P.kmask_mul, s[i]);
+                prefill_add_mask(P, mk, k0, s);
             }
-            if (P.qkmask != nullptr) {
+            if (MASK == 2) {
                 // additive [Sq, Skv] mask tensor: each thread reads its own row's values for this tile (-inf entries give
                 // -inf scores, which the code below treats like keys outside a window); no tile can be skipped
                 const float* mr = P.qkmask + (long long)min(qi, P.Sq - 1) * P.qkmask_stride;
-#pragma unroll
-                for (int i = 0; i < PF_CPT; ++i) s[i] = fmaf(__ldg(mr + min(k0 + i, P.Skv - 1)), P.kmask_mul, s[i]);
+                prefill_add_mask(P, mr, k0, s);
             }
             if (k0 + PF_CPT - 1 > k_limit || k0 < k_first) {  // diagonal, ragged or window-edge tile: mask in the raw domain
 #pragma unroll
@@ -296,14 +337,18 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
                 if (!ok) break;
                 pmax = fmaxf(pmax, xch[((j & 1) * 2 + (half ^ 1)) * 128 + row]);
             }
-            const float tmax = pmax * c;  // scale > 0
+            const float tmax = MASK ? pmax : pmax * c;  // scale > 0
             // lazy rescale: keep the reference max until the true max has moved by more than the threshold
-            const float m_new = (tmax > m_ref + PF_RESCALE_THRESHOLD) ? tmax : m_ref;  // also taken on the first tile
+            const float m_new = (tmax > m_ref + thr) ? tmax : m_ref;  // also taken on the first tile
             // A row whose keys so far are all outside its window keeps m = -inf: its weights are exp2(-inf - 0) = 0
             // and its O row stays 0, without a NaN from (-inf) - (-inf).
-            const float alpha = (m_new == -INFINITY) ? 1.0f : fast_exp2(m_ref - m_new);  // 1 when unchanged, 0 on a row's first tile
+            const float alpha = (m_new == -INFINITY) ? 1.0f : fast_exp2((m_ref - m_new) * m_unit);  // 1 when unchanged, 0 on a row's first tile
             m_ref = m_new;
-            const float m_sub = (m_ref == -INFINITY) ? 0.0f : m_ref;
+            float m_sub = (m_ref == -INFINITY) ? 0.0f : m_ref;
+            if (MASK) {
+                prefill_subtract(m_sub, s);
+                m_sub = 0.0f;
+            }
             const float2 c2 = make_float2(c, c), nm2 = make_float2(-m_sub, -m_sub);
             float2 ps0 = make_float2(0.0f, 0.0f), ps1 = make_float2(0.0f, 0.0f);
 #pragma unroll
@@ -420,10 +465,10 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
             for (int k = 0; k < parts; ++k) M = fmaxf(M, part_ml[k * 128 + row].x);
             for (int k = 0; k < parts; ++k) {
                 const float2 ml = part_ml[k * 128 + row];
-                if (ml.x != -INFINITY) L += ml.y * fast_exp2(ml.x - M);
+                if (ml.x != -INFINITY) L += ml.y * fast_exp2((ml.x - M) * m_unit);
             }
             // (a row no part saw a key for: L = 0, and 0 * inf = NaN as without parts)
-            f = (m_ref == -INFINITY ? 0.0f : fast_exp2(m_ref - M)) * (1.0f / L);
+            f = (m_ref == -INFINITY ? 0.0f : fast_exp2((m_ref - M) * m_unit)) * (1.0f / L);
             tc_fence_after();
         }
         auto scaled = [&](int col, float (&v)[16]) {  // 16 columns of this part's O, scaled; 0 (or NaN) where it saw no tile

@@ -23,7 +23,7 @@ def _rows(rng, n, keys):
         elif kind == 1: m[i] = -np.inf
         elif kind == 2: m[i] = np.where(rng.random(keys) < 0.5, LOWEST, -np.inf); m[i, keys // 2] = LOWEST
         elif kind == 3: m[i] = np.where(rng.random(keys) < 0.5, LOWEST, 0.0); m[i, keys // 3] = 0.0
-        elif kind == 4: m[i] = -2.4e38
+        elif kind == 4: m[i] = -2.4e38 if i % 16 == 4 else -1e9
         elif kind == 5: m[i] = -1e4
         elif kind == 6: m[i] = LOWEST; m[i, -1] = 0.5
         else: m[i] = rng.choice(np.array([0.0, LOWEST, -np.inf, -1e4, 1.0], np.float32), keys); m[i, 0] = 0.0
@@ -56,3 +56,12 @@ def _check(device, dtype, D, kind, B, Hq, Hkv, Sq, Skv, max_tol, mean_tol):
 def test_f32_accuracy_kernels(device, dtype, D, kind, B, Sq, Skv):
     """Warp MMAs on f32 and on 16-bit tensors, and the general kernel (head_dim above 128 or not a multiple of 8)."""
     _check(device, dtype, D, kind, B, 4, 2, Sq, Skv, 2e-5, 2e-6)
+
+
+@pytest.mark.parametrize("kind,B,Hq,Hkv,Sq,Skv", [
+    ("tensor", 1, 4, 2, 72, 200), ("key", 8, 4, 2, 40, 131), ("tensor", 1, 2, 1, 130, 1100), ("key", 8, 1, 1, 70, 1300),  # a tile's keys on one CTA, on several
+    ("key", 8, 20, 4, 400, 400),                                                                                         # two query tiles per CTA
+])
+@pytest.mark.parametrize("dtype", [1, 2])
+def test_tcgen05_kernels(device, dtype, kind, B, Hq, Hkv, Sq, Skv):
+    _check(device, dtype, 128, kind, B, Hq, Hkv, Sq, Skv, 2e-3, 2e-4)
