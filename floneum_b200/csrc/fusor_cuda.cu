@@ -40,11 +40,12 @@ using namespace fusor;
 // cudaFree pair with the device-wide wait inside cudaFree cost 0.4 to 3 ms of host time, many times the kernels (back to back:
 // attention of a 777-token prompt 0.8 to 3 ms, 29 us with kept buffers; a prefill of B4 S4096 with its 268 MB result 1.5 ms
 // and 0.60 ms).  A freed buffer may still be read by work on ANY stream (the library's, torch's), which is why cudaFree waits
-// for the whole device; here freed buffers wait together: they are handed out again only after a cudaDeviceSynchronize that
-// came after their release.  That wait is made when a buffer of the size is among them and the context's own stream has
-// nothing to do (a program that reads its results back is there already), or enough of the size are waiting to spread its
-// cost.  Kept: at most a 64th of the device's memory; larger buffers than a quarter of that go straight to cudaMalloc /
-// cudaFree, and so does everything while the context's stream is being captured (a graph keeps the addresses it saw).
+// for the whole device; here freed buffers wait together: they are handed out again only after a device-wide wait that came
+// after their release.  That wait is made when a buffer of the size is among them and the context's own stream has nothing to
+// do (a program that reads its results back is there already), or enough of the size are waiting to spread its cost.  It is
+// made by a cudaFree (see settle).  Kept: at most a 64th of the device's memory; larger buffers than a quarter of that go
+// straight to cudaMalloc / cudaFree, and so does everything while the context's stream is being captured (a graph keeps the
+// addresses it saw).
 class BufferPool {
   public:
     void set_limit(size_t bytes) { limit_ = bytes; }
@@ -72,7 +73,7 @@ class BufferPool {
         cudaError_t e = cudaMalloc(out, size);
         if (e == cudaErrorMemoryAllocation) {
             cudaGetLastError();
-            if (settle() == cudaSuccess) trim(0);
+            free_kept();
             e = cudaMalloc(out, size);
         }
         if (e == cudaSuccess) live_[*out] = size;
@@ -111,7 +112,7 @@ class BufferPool {
             std::lock_guard<std::mutex> lock(mutex_);
             if (kept_ == 0) return e;
             cudaGetLastError();
-            if (settle() == cudaSuccess) trim(0);
+            free_kept();
             e = cudaMalloc(out, bytes);
         }
         return e;
@@ -119,7 +120,9 @@ class BufferPool {
 
     void drain() {  // gives everything kept back
         std::lock_guard<std::mutex> lock(mutex_);
-        if (kept_ > 0 && settle() == cudaSuccess) trim(0);
+        free_kept();
+        if (anchor_) cudaFree(anchor_);
+        anchor_ = nullptr;
     }
 
   private:
@@ -142,8 +145,18 @@ class BufferPool {
         ready_.erase(it);
         return true;
     }
+    // The device-wide wait: cudaFree of a few bytes, which waits for the work of every stream, as it does for any buffer.
+    // cudaDeviceSynchronize waits as well, but while another thread captures a graph in a mode that allows cudaMalloc and
+    // cudaFree it fails and ends that capture too.  A small buffer held on to keeps the driver's block of small allocations
+    // mapped: the pair takes 5 us beside it and 610 us without.
     cudaError_t settle() {
-        const cudaError_t e = cudaDeviceSynchronize();
+        if (!anchor_) {
+            const cudaError_t e = cudaMalloc(&anchor_, 256);
+            if (e != cudaSuccess) return e;
+        }
+        void* p = nullptr;
+        cudaError_t e = cudaMalloc(&p, 256);
+        if (e == cudaSuccess) e = cudaFree(p);
         if (e != cudaSuccess) return e;
         for (const Block& b : freed_) ready_.emplace(b.size, b.ptr);
         freed_.clear();
@@ -158,9 +171,19 @@ class BufferPool {
             ready_.erase(it);
         }
     }
+    void free_kept() {  // all of them; cudaFree waits for those that may still be read
+        trim(0);
+        for (const Block& b : freed_) {
+            cudaFree(b.ptr);
+            kept_ -= b.size;
+        }
+        freed_.clear();
+        freed_of_.clear();
+    }
 
     std::mutex mutex_;
     size_t limit_ = 0, kept_ = 0;
+    void* anchor_ = nullptr;
     std::unordered_map<void*, size_t> live_;       // handed out
     std::vector<Block> freed_;                     // released since the last device-wide wait
     std::unordered_map<size_t, size_t> freed_of_;  // how many of a size

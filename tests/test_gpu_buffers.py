@@ -48,3 +48,43 @@ def test_buffers_come_back_and_a_second_free_is_refused(device):
     assert len(set(held)) == 50
     for q in held:
         device.free(q)
+
+
+@pytest.mark.parametrize("mode", ["thread_local", "relaxed"])
+def test_buffers_while_another_thread_captures_a_graph(device, mode):
+    """Allocation and release go on, and the other thread's capture survives them (both modes allow cudaMalloc and cudaFree)."""
+    import threading
+    import torch
+    import floneum_b200 as fb
+    x = torch.ones(1024, device="cuda")
+    torch.cuda.synchronize()
+    begun, done, got = threading.Event(), threading.Event(), []
+
+    def capture():
+        try:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.stream(torch.cuda.Stream()):
+                graph.capture_begin(capture_error_mode=mode)
+                y = x * 2
+                begun.set()
+                done.wait(60)
+                y = y + 1
+                graph.capture_end()
+            graph.replay()
+            torch.cuda.synchronize()
+            got.append(float(y[0]))
+        except Exception as e:
+            got.append(e)
+            begun.set()
+
+    t = threading.Thread(target=capture)
+    t.start()
+    begun.wait(60)
+    try:
+        for _ in range(600):  # enough releases for several rounds of reuse
+            a, b = fb.Tensor.empty(device, (1 << 16,)), fb.Tensor.empty(device, (1 << 16,))
+            del a, b
+    finally:
+        done.set()
+        t.join()
+    assert got == [3.0]
