@@ -48,7 +48,11 @@ using namespace fusor;
 // addresses it saw).
 class BufferPool {
   public:
-    void set_limit(size_t bytes) { limit_ = bytes; }
+    using AddressRange = CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr);
+    void init(size_t limit, AddressRange range) {
+        limit_ = limit;
+        range_ = range;
+    }
 
     cudaError_t alloc(size_t bytes, cudaStream_t stream, void** out) {
         const size_t size = rounded(bytes);
@@ -95,6 +99,11 @@ class BufferPool {
         }
         const size_t size = it->second;
         live_.erase(it);
+        // A buffer that was freed elsewhere (through another context, or by cudaFree) is still on record here; whoever has got its
+        // address since may release it here too.  What is kept is therefore of the size that the driver knows.
+        CUdeviceptr base = 0;
+        size_t bytes = 0;
+        if (range_(&base, &bytes, reinterpret_cast<CUdeviceptr>(p)) != CUDA_SUCCESS || base != reinterpret_cast<CUdeviceptr>(p) || bytes < size) return NOT_KEPT;
         if (kept_ + size > limit_) {
             if (settle() == cudaSuccess) trim(limit_ / 2);
             if (kept_ + size > limit_) return NOT_KEPT;
@@ -183,6 +192,7 @@ class BufferPool {
 
     std::mutex mutex_;
     size_t limit_ = 0, kept_ = 0;
+    AddressRange range_ = nullptr;
     void* anchor_ = nullptr;
     std::unordered_map<void*, size_t> live_;       // handed out
     std::vector<Block> freed_;                     // released since the last device-wide wait
@@ -300,7 +310,6 @@ extern "C" int32_t fusor_cuda_ctx_create(int32_t device, void* stream, fusor_cud
     fusor_cuda_ctx* ctx = new fusor_cuda_ctx();
     ctx->device = device;
     ctx->num_sms = prop.multiProcessorCount;
-    ctx->pool.set_limit(prop.totalGlobalMem / 64);
     if (stream) {
         ctx->stream = static_cast<cudaStream_t>(stream);
     } else {
@@ -325,6 +334,12 @@ extern "C" int32_t fusor_cuda_ctx_create(int32_t device, void* stream, fusor_cud
         return fail(nullptr, FUSOR_CUDA_CUDA_ERROR, "cuTensorMapEncodeTiled is not available in this driver");
     }
     ctx->encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
+    void* range = nullptr;
+    if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &range, cudaEnableDefault, &qres) != cudaSuccess || !range) {
+        fusor_cuda_ctx_destroy(ctx);
+        return fail(nullptr, FUSOR_CUDA_CUDA_ERROR, "cuMemGetAddressRange is not available in this driver");
+    }
+    ctx->pool.init(prop.totalGlobalMem / 64, reinterpret_cast<BufferPool::AddressRange>(range));
     // opt in to large dynamic shared memory once per context (each call is checked by its own return value: a kernel
     // whose static shared memory pushes the sum over the limit must fail here, not at its first launch)
     struct { const void* fn; int bytes; const char* name; } opt_in[] = {
