@@ -1811,8 +1811,8 @@ extern "C" int32_t fusor_cuda_exchange_create(fusor_cuda_ctx* ctx, int32_t world
     ex->ctx = ctx; ex->world = world; ex->rank = rank; ex->slot_floats = (size_t)slot_floats;
     ex->flags_off = align256(2 * (size_t)world * ex->slot_floats * 4);
     const size_t bytes = ex->flags_off + align256(2 * (size_t)world * 8);
-    if (cudaMalloc(&ex->base, bytes) != cudaSuccess || cudaMemset(ex->base, 0, bytes) != cudaSuccess ||
-        cudaMalloc(&ex->done, 256) != cudaSuccess || cudaMemset(ex->done, 0, 256) != cudaSuccess) {
+    if (ctx->pool.plain(bytes, &ex->base) != cudaSuccess || cudaMemset(ex->base, 0, bytes) != cudaSuccess ||
+        ctx->pool.plain(256, reinterpret_cast<void**>(&ex->done)) != cudaSuccess || cudaMemset(ex->done, 0, 256) != cudaSuccess) {
         cudaError_t e = cudaGetLastError();
         if (ex->base) cudaFree(ex->base);
         if (ex->done) cudaFree(ex->done);
@@ -2046,6 +2046,7 @@ extern "C" int32_t fusor_cuda_comm_init(fusor_cuda_ctx* ctx, const void* id128, 
     std::memcpy(&id, id128, 128);
     ncclConfig_t config = NCCL_CONFIG_INITIALIZER;
     config.blocking = 0;  // every call returns at once; completion is polled against the caller's deadline
+    ctx->pool.drain();    // NCCL allocates for itself
     const ncclResult_t r = api->CommInitRankConfig(&cm->comm, world, id, rank, &config);
     if (r != ncclSuccess && r != ncclInProgress) {
         const int32_t rc = fail(ctx, FUSOR_CUDA_NCCL_ERROR, "ncclCommInitRankConfig: %s", api->GetErrorString(r));

@@ -133,3 +133,26 @@ def test_a_buffer_freed_through_another_context_leaves_no_size_behind(device):
     finally:
         for q in again:
             device.free(q)
+
+
+def test_the_exchange_buffer_may_use_what_is_kept(device):
+    """On a full GPU the bytes that the pool keeps are given back before an allocation of the library fails."""
+    import gc
+    import torch
+    import floneum_b200 as fb
+    from floneum_b200 import _lib
+    L, ex = _lib.load(), ctypes.c_void_p()
+    gc.collect()
+    torch.cuda.empty_cache()
+    mine = fb.Device.gpu(0)
+    held = [mine.alloc(500 << 20) for _ in range(4)]
+    for p in held:
+        mine.free(p)
+    rest = torch.empty(torch.cuda.mem_get_info()[0] - (400 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        assert torch.cuda.mem_get_info()[0] < 900 << 20
+        _lib.check(L.fusor_cuda_exchange_create(mine.handle, 1, 0, 1 << 27, ctypes.byref(ex)), mine.handle)  # two parities of 512 MB
+        L.fusor_cuda_exchange_destroy(ex)
+    finally:
+        del rest
+        torch.cuda.empty_cache()
