@@ -496,6 +496,13 @@ extern "C" int32_t fusor_cuda_buffer_free(fusor_cuda_ctx* ctx, void* device_ptr)
     CUDA_TRY(ctx, cudaFree(device_ptr));
     return FUSOR_CUDA_OK;
 }
+extern "C" int32_t fusor_cuda_buffer_trim(fusor_cuda_ctx* ctx) {
+    if (!ctx) return fail(nullptr, FUSOR_CUDA_INVALID_ARGUMENT, "ctx is null");
+    DeviceGuard g(ctx->device);
+    if (capturing(ctx)) CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));  // refused, as cudaFree is
+    ctx->pool.drain();
+    return FUSOR_CUDA_OK;
+}
 extern "C" int32_t fusor_cuda_buffer_upload(fusor_cuda_ctx* ctx, void* dst, const void* src, size_t bytes) {
     if (!ctx || (bytes && (!dst || !src))) return fail(ctx, FUSOR_CUDA_INVALID_ARGUMENT, "null argument");
     DeviceGuard g(ctx->device);

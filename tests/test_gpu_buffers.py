@@ -156,3 +156,19 @@ def test_the_exchange_buffer_may_use_what_is_kept(device):
     finally:
         del rest
         torch.cuda.empty_cache()
+
+
+def test_kept_buffers_can_be_asked_back(device):
+    import torch
+    import floneum_b200 as fb
+    mine = fb.Device.gpu(0)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    held = [mine.alloc(500 << 20) for _ in range(4)]
+    for p in held:
+        mine.free(p)
+    assert torch.cuda.mem_get_info()[0] < before - (1 << 30)  # kept
+    mine.trim()
+    assert torch.cuda.mem_get_info()[0] > before - (64 << 20)
+    q = mine.alloc(500 << 20)
+    mine.free(q)
