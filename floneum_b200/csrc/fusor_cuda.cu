@@ -743,16 +743,18 @@ static int32_t launch_mma(fusor_cuda_ctx* ctx, const AttnShape& S, const fusor_c
 
 // The softmax weights are kept in f16 against an f16 copy of V (the kernels fall back to bf16 weights and the bf16 V on
 // the device when some |v| does not fit f16).
+// `call_heads`: (batch, query head) pairs that the choice of the kernel counts, those of the whole call where this is a part of
+// it: the bits of a head's result then do not depend on how a call was cut up.
 static int32_t launch_prefill(fusor_cuda_ctx* ctx, const AttnShape& S, const fusor_cuda_tensor4* q,
                               const fusor_cuda_tensor4* k, const fusor_cuda_tensor4* v, float scale, int32_t mask_kind,
-                              const fusor_cuda_tensor4* out, int window = 0, const fusor_cuda_tensor2* key_mask = nullptr,
-                              const fusor_cuda_tensor2* qk_mask = nullptr) {
+                              const fusor_cuda_tensor4* out, int window, const fusor_cuda_tensor2* key_mask,
+                              const fusor_cuda_tensor2* qk_mask, long long call_heads) {
     // Two query tiles per CTA with 128-key blocks once the 256-row items outnumber the SMs; below that its CTAs each have one
     // item and the call lasts as long as the longest, which 128-row tiles on twice the CTAs finish sooner (H32/8 causal, us,
     // two tiles / one: S512 15.9 / 12.7, S1000 24.1 / 20.9, S1500 33.0 / 34.4 with 192 items; H8/8 S4096 67 / 60; B4 S300
     // 21.3 / 18.1, where every second item is half empty).  Calls with an additive [Sq, Skv] mask tensor always take the 64-key
     // kernel (each softmax thread reads a row of mask values per tile: it has the registers for that).
-    const long long items = (long long)((S.Sq + P2_ROWS - 1) / P2_ROWS) * S.Hq * S.B;
+    const long long items = (long long)((S.Sq + P2_ROWS - 1) / P2_ROWS) * call_heads;
     const bool two_tiles = S.Sq > P2_ROWS + P2_BM && items > ctx->num_sms && qk_mask == nullptr;
     const int kv_rows = two_tiles ? P2_BN : PF_BN;
     const bool in_f16 = q->dtype == FUSOR_CUDA_F16;  // f16 tensors need no copy of V: the weights are f16 against V itself
@@ -815,7 +817,7 @@ static int32_t launch_prefill(fusor_cuda_ctx* ctx, const AttnShape& S, const fus
     // the longest row of tiles has to be 16 for two parts, and a part keeps more than 4.5.
     const long long longest = (std::min(S.Skv, P.window > 0 ? P.window + PF_BM : S.Skv) + PF_BN - 1) / PF_BN;
     int parts = 1;
-    while (parts < PF_MAX_SPLIT && grid * parts * 2 <= 2ll * ctx->num_sms && longest > (parts == 1 ? 15 : 9ll * parts)) parts *= 2;
+    while (parts < PF_MAX_SPLIT && P.n_q_tiles * call_heads * parts * 2 <= 2ll * ctx->num_sms && longest > (parts == 1 ? 15 : 9ll * parts)) parts *= 2;
     if (parts > 1) {
         cudaLaunchAttribute attr;
         const cudaLaunchConfig_t cfg = cluster_config(ctx, (unsigned)(grid * parts), (unsigned)parts, PF_THREADS, PF_SMEM_BYTES, &attr);
@@ -827,18 +829,24 @@ static int32_t launch_prefill(fusor_cuda_ctx* ctx, const AttnShape& S, const fus
     return launch_check(ctx, "prefill_sm100_kernel");
 }
 
-extern "C" int32_t fusor_cuda_flash_attention(fusor_cuda_ctx* ctx, const fusor_cuda_tensor4* q, const fusor_cuda_tensor4* k,
-                                              const fusor_cuda_tensor4* v, float scale, const fusor_cuda_tensor2* mask,
-                                              int32_t mask_kind, int32_t window, const fusor_cuda_tensor4* out) {
+// A call, or (call_heads > 0) a part of one with that many (batch, query head) pairs.
+static int32_t flash_attention(fusor_cuda_ctx* ctx, const fusor_cuda_tensor4* q, const fusor_cuda_tensor4* k, const fusor_cuda_tensor4* v, float scale,
+                               const fusor_cuda_tensor2* mask, int32_t mask_kind, int32_t window, const fusor_cuda_tensor4* out, long long call_heads) {
     AttnShape S;
     TRY(validate_attention(ctx, q, k, v, mask, mask_kind, window, out, &S));
     DeviceGuard g(ctx->device);
     if (prefill_eligible(S, q, k, v, scale, mask_kind, out, mask))
         return launch_prefill(ctx, S, q, k, v, scale, mask_kind, out, window,
                               mask_kind == FUSOR_CUDA_MASK_BATCH_KEY ? mask : nullptr,
-                              mask_kind == FUSOR_CUDA_MASK_QK ? mask : nullptr);
+                              mask_kind == FUSOR_CUDA_MASK_QK ? mask : nullptr, call_heads > 0 ? call_heads : (long long)S.B * S.Hq);
     if (mma_eligible(S, q, k, v, scale, out)) return launch_mma(ctx, S, q, k, v, scale, mask, mask_kind, window, out);
     return launch_general(ctx, S, q, k, v, scale, mask, mask_kind, window, out);
+}
+
+extern "C" int32_t fusor_cuda_flash_attention(fusor_cuda_ctx* ctx, const fusor_cuda_tensor4* q, const fusor_cuda_tensor4* k,
+                                              const fusor_cuda_tensor4* v, float scale, const fusor_cuda_tensor2* mask,
+                                              int32_t mask_kind, int32_t window, const fusor_cuda_tensor4* out) {
+    return flash_attention(ctx, q, k, v, scale, mask, mask_kind, window, out, 0);
 }
 
 extern "C" int32_t fusor_cuda_flash_attention_general(fusor_cuda_ctx* ctx, const fusor_cuda_tensor4* q,
@@ -1032,7 +1040,7 @@ extern "C" int32_t fusor_cuda_flash_attention_host(fusor_cuda_ctx* ctx, const fu
             cudaMemcpyAsync(cv.data, (const uint8_t*)v->data + ko * vs, kv_chunk * vs, cudaMemcpyHostToDevice, ctx->h2d_stream);
             cudaEventRecord(in_done, ctx->h2d_stream);
             cudaStreamWaitEvent(ctx->stream, in_done, 0);
-            rc = fusor_cuda_flash_attention(ctx, &cq, &ck, &cv, scale, nullptr, mask_kind, window, &co);
+            rc = flash_attention(ctx, &cq, &ck, &cv, scale, nullptr, mask_kind, window, &co, (long long)S.B * S.Hq);
             if (rc != FUSOR_CUDA_OK) break;
             cudaEventRecord(k_done, ctx->stream);
             cudaStreamWaitEvent(ctx->d2h_stream, k_done, 0);
