@@ -596,6 +596,11 @@ static int32_t validate_attention(fusor_cuda_ctx* ctx, const fusor_cuda_tensor4*
     return FUSOR_CUDA_OK;
 }
 
+// the limit of every call that the tcgen05 kernels do not take
+static int32_t check_heads(fusor_cuda_ctx* ctx, const AttnShape& S) {
+    return S.Hq > 65535 || S.B > 65535 ? fail(ctx, FUSOR_CUDA_UNSUPPORTED, "more than 65535 heads or batches") : FUSOR_CUDA_OK;
+}
+
 // =============================================================================== attention: launches
 static int32_t launch_general(fusor_cuda_ctx* ctx, const AttnShape& S, const fusor_cuda_tensor4* q,
                               const fusor_cuda_tensor4* k, const fusor_cuda_tensor4* v, float scale,
@@ -815,7 +820,7 @@ static int32_t launch_prefill(fusor_cuda_ctx* ctx, const AttnShape& S, const fus
     }
     // Few tiles: parts of the keys on up to 8 CTAs each, two CTAs per SM.  The merge costs as much as four to six key tiles, so
     // the longest row of tiles has to be 16 for two parts, and a part keeps more than 4.5.
-    const long long longest = (std::min(S.Skv, P.window > 0 ? P.window + PF_BM : S.Skv) + PF_BN - 1) / PF_BN;
+    const long long longest = (std::min(S.Skv, P.window > 0 && P.window < S.Skv ? P.window + PF_BM : S.Skv) + PF_BN - 1) / PF_BN;
     int parts = 1;
     while (parts < PF_MAX_SPLIT && P.n_q_tiles * call_heads * parts * 2 <= 2ll * ctx->num_sms && longest > (parts == 1 ? 15 : 9ll * parts)) parts *= 2;
     if (parts > 1) {
@@ -839,6 +844,7 @@ static int32_t flash_attention(fusor_cuda_ctx* ctx, const fusor_cuda_tensor4* q,
         return launch_prefill(ctx, S, q, k, v, scale, mask_kind, out, window,
                               mask_kind == FUSOR_CUDA_MASK_BATCH_KEY ? mask : nullptr,
                               mask_kind == FUSOR_CUDA_MASK_QK ? mask : nullptr, call_heads > 0 ? call_heads : (long long)S.B * S.Hq);
+    TRY(check_heads(ctx, S));
     if (mma_eligible(S, q, k, v, scale, out)) return launch_mma(ctx, S, q, k, v, scale, mask, mask_kind, window, out);
     return launch_general(ctx, S, q, k, v, scale, mask, mask_kind, window, out);
 }
@@ -856,6 +862,7 @@ extern "C" int32_t fusor_cuda_flash_attention_general(fusor_cuda_ctx* ctx, const
     AttnShape S;
     TRY(validate_attention(ctx, q, k, v, mask, mask_kind, window, out, &S));
     DeviceGuard g(ctx->device);
+    TRY(check_heads(ctx, S));
     return launch_general(ctx, S, q, k, v, scale, mask, mask_kind, window, out);
 }
 
@@ -921,11 +928,12 @@ extern "C" int32_t fusor_cuda_attention_out_proj(fusor_cuda_ctx* ctx, const fuso
         return fail(ctx, FUSOR_CUDA_UNSUPPORTED, "the output projection takes bf16 attention output and bf16 weights and writes f32 or bf16");
     if (D % OP_BK != 0) return fail(ctx, FUSOR_CUDA_UNSUPPORTED, "head_dim must be a multiple of %d", OP_BK);
     if (!tma_view_ok(attn)) return fail(ctx, FUSOR_CUDA_UNSUPPORTED, "attention output view is not 16-byte aligned");
-    if (weight->stride[3] != 1 || weight->stride[2] % 8 != 0 || reinterpret_cast<uintptr_t>(weight->data) % 16)
-        return fail(ctx, FUSOR_CUDA_UNSUPPORTED, "weight rows must be contiguous and 16-byte aligned");
+    if (weight->stride[3] != 1 || weight->stride[2] % 8 != 0 || (N > 1 && weight->stride[2] < 0) || reinterpret_cast<uintptr_t>(weight->data) % 16)
+        return fail(ctx, FUSOR_CUDA_UNSUPPORTED, "weight rows must be contiguous, in ascending order and 16-byte aligned");
     const int al = out->dtype == FUSOR_CUDA_F32 ? 4 : 8;
-    if (out->stride[3] != 1 || out->stride[2] % al != 0 || (B > 1 && out->stride[0] % al != 0) || reinterpret_cast<uintptr_t>(out->data) % 16)
-        return fail(ctx, FUSOR_CUDA_UNSUPPORTED, "out rows must be contiguous and 16-byte aligned");
+    if (out->stride[3] != 1 || out->stride[2] % al != 0 || (S > 1 && out->stride[2] < 0) || (B > 1 && (out->stride[0] % al != 0 || out->stride[0] < 0)) ||
+        reinterpret_cast<uintptr_t>(out->data) % 16)
+        return fail(ctx, FUSOR_CUDA_UNSUPPORTED, "out rows must be contiguous, in ascending order and 16-byte aligned");
     if (bias && reinterpret_cast<uintptr_t>(bias) % 4) return fail(ctx, FUSOR_CUDA_INVALID_ARGUMENT, "bias is misaligned");
     DeviceGuard g(ctx->device);
     fusor_cuda_tensor4 w4 = *weight;
