@@ -189,13 +189,27 @@ __device__ __forceinline__ void decode_load_q(const DecodeParams& P, int b, int 
     }
 }
 
+// The first n rows of a V tile in shared memory become zero: rows that have been evicted from the front of a sequence's first
+// page.  Their weight is zero, but zero times a value that is not finite would still reach the sum.  Whole warp.
+template <int D>
+__device__ __forceinline__ void decode_clear_rows(uint32_t vb, int n, int lane) {
+#pragma unroll
+    for (int half = 0; half < D / 64; ++half)
+        for (int i = lane; i < n * 8; i += 32)
+            asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(vb + half * (DEC_PT * 128) + i * 16), "r"(0) : "memory");
+    fence_proxy_async_smem();  // the slot's next TMA copy comes after these stores
+    __syncwarp();
+}
+
 // One page (16 tokens from tok0 on, of which 0 .. len - 1 exist) into a warp's running state: K tile at shared address kb, V at vb.
+// Whole warp; the tile of a first page with evicted rows (tok0 < 0) is changed.
 template <int D>
 __device__ __forceinline__ void decode_page(uint32_t kb, uint32_t vb, const uint32_t (&qa)[D / 16][2], int tok0, int len, float scale_log2,
                                             int lane, float& m_run, float& l_run, float (&o)[D / 8][4]) {
     constexpr int HALF_BYTES = DEC_PT * 128;      // one 64-column half of a page tile
     const int cq = (lane & 3) * 2;                // column pair inside an 8-wide tile
     const int lm_j = lane >> 3, lm_r = lane & 7;  // ldmatrix lane geometry
+    if (tok0 < 0) decode_clear_rows<D>(vb, -tok0, lane);  // (here: after the softmax it would hold back the loads of V, 7 % of a batch)
     // ---- S = Q K^T for 16 tokens (two 8-token tiles)
     float s[2][4];
 #pragma unroll

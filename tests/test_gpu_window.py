@@ -98,3 +98,25 @@ def test_lengths_reach_the_device_with_and_without_a_launch_that_carries_them(de
         got = cache.decode(T(q), 0.125).as_slice()
         assert_close(got, O.flash_attention(q, k[:, :, lo:at], k[:, :, lo:at], 0.125), what=f"{lo}..{at}")
         assert np.array_equal(cache.gather(B, at - lo)[0].as_slice(), k[:, :, lo:at])
+
+
+@pytest.mark.parametrize("D,window", [(128, 40), (64, 40), (128, 200), (64, 200)])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_an_evicted_row_has_no_part_in_the_result(device, D, window, bad):
+    """A value that is not finite leaves with its row, whether the decode runs in one cluster per head or on the even deal."""
+    fb = _fb()
+    rng = np.random.default_rng(D + window)
+    B, Hq, Hkv, n = 1, 4, 2, window + 20
+    k, v = (O.bf16_round(rng.standard_normal((B, Hkv, n, D), dtype=np.float32)) for _ in range(2))
+    q = O.bf16_round(rng.standard_normal((B, Hq, 1, D), dtype=np.float32))
+    v[0, 0, 3, 1], v[0, 1, 17, 2] = bad, bad
+    T = lambda a: fb.Tensor.from_slice(device, a.shape, np.ascontiguousarray(a))
+    cache, scale = fb.KvCache.new(2, window), float(D ** -0.5)
+    cache.append(device, T(k[:, :, :window]), T(v[:, :, :window]))
+    for at in range(window + 1, n + 1):
+        ck, cv = cache.append(device, T(k[:, :, at - 1:at]), T(v[:, :, at - 1:at]))
+        lo = at - window
+        got = T(q).flash_attention(ck, cv, scale).as_slice()
+        assert np.isfinite(got[:, :2]).all() == (lo > 3) and np.isfinite(got[:, 2:]).all() == (lo > 17), lo
+        if lo > 17:
+            assert_close(got, O.flash_attention(q, k[:, :, lo:at], v[:, :, lo:at], scale), what=f"{at} tokens")
