@@ -50,6 +50,7 @@ SIGNATURES = {
     "fusor_cuda_launch_count": (c_int64, [c_void_p]),
     "fusor_cuda_buffer_alloc": (c_int32, [c_void_p, c_size_t, POINTER(c_void_p)]),
     "fusor_cuda_buffer_free": (c_int32, [c_void_p, c_void_p]),
+    "fusor_cuda_buffer_trim": (c_int32, [c_void_p]),
     "fusor_cuda_buffer_upload": (c_int32, [c_void_p, c_void_p, c_void_p, c_size_t]),
     "fusor_cuda_buffer_download": (c_int32, [c_void_p, c_void_p, c_void_p, c_size_t]),
     "fusor_cuda_cast": (c_int32, [c_void_p, c_void_p, c_int32, c_void_p, c_int32, c_int64]),

@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(AM_THREADS, DP <= 64 ? 3 : 2) attn_mma16_kerne
             }
         }
         if (kt + AM_BN > P.Skv || (causal && kt + AM_BN - 1 > q0 + warp * 16 + offset) ||
-            (P.mask_kind == 4 && kt + P.window <= q0 + warp * 16 + 15 + offset)) {
+            (P.mask_kind == 4 && kt <= q0 + warp * 16 + 15 + offset - P.window)) {
 #pragma unroll
             for (int nt = 0; nt < AM_BN / 8; ++nt)
 #pragma unroll

@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(AM_THREADS, DP <= 64 ? 2 : 1) attn_mma32_kerne
             }
         }
         if (kt + BN > P.Skv || (causal && kt + BN - 1 > q0 + warp * 16 + offset) ||
-            (P.mask_kind == 4 && kt + P.window <= q0 + warp * 16 + 15 + offset)) {
+            (P.mask_kind == 4 && kt <= q0 + warp * 16 + 15 + offset - P.window)) {
 #pragma unroll
             for (int nt = 0; nt < BN / 8; ++nt)
 #pragma unroll

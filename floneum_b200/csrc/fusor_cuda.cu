@@ -48,7 +48,11 @@ using namespace fusor;
 // addresses it saw).
 class BufferPool {
   public:
-    void set_limit(size_t bytes) { limit_ = bytes; }
+    using AddressRange = CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr);
+    void init(size_t limit, AddressRange range) {
+        limit_ = limit;
+        range_ = range;
+    }
 
     cudaError_t alloc(size_t bytes, cudaStream_t stream, void** out) {
         const size_t size = rounded(bytes);
@@ -95,6 +99,11 @@ class BufferPool {
         }
         const size_t size = it->second;
         live_.erase(it);
+        // A buffer that was freed elsewhere (through another context, or by cudaFree) is still on record here; whoever has got its
+        // address since may release it here too.  What is kept is therefore of the size that the driver knows.
+        CUdeviceptr base = 0;
+        size_t bytes = 0;
+        if (range_(&base, &bytes, reinterpret_cast<CUdeviceptr>(p)) != CUDA_SUCCESS || base != reinterpret_cast<CUdeviceptr>(p) || bytes < size) return NOT_KEPT;
         if (kept_ + size > limit_) {
             if (settle() == cudaSuccess) trim(limit_ / 2);
             if (kept_ + size > limit_) return NOT_KEPT;
@@ -183,6 +192,7 @@ class BufferPool {
 
     std::mutex mutex_;
     size_t limit_ = 0, kept_ = 0;
+    AddressRange range_ = nullptr;
     void* anchor_ = nullptr;
     std::unordered_map<void*, size_t> live_;       // handed out
     std::vector<Block> freed_;                     // released since the last device-wide wait
@@ -300,7 +310,6 @@ extern "C" int32_t fusor_cuda_ctx_create(int32_t device, void* stream, fusor_cud
     fusor_cuda_ctx* ctx = new fusor_cuda_ctx();
     ctx->device = device;
     ctx->num_sms = prop.multiProcessorCount;
-    ctx->pool.set_limit(prop.totalGlobalMem / 64);
     if (stream) {
         ctx->stream = static_cast<cudaStream_t>(stream);
     } else {
@@ -325,6 +334,12 @@ extern "C" int32_t fusor_cuda_ctx_create(int32_t device, void* stream, fusor_cud
         return fail(nullptr, FUSOR_CUDA_CUDA_ERROR, "cuTensorMapEncodeTiled is not available in this driver");
     }
     ctx->encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
+    void* range = nullptr;
+    if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &range, cudaEnableDefault, &qres) != cudaSuccess || !range) {
+        fusor_cuda_ctx_destroy(ctx);
+        return fail(nullptr, FUSOR_CUDA_CUDA_ERROR, "cuMemGetAddressRange is not available in this driver");
+    }
+    ctx->pool.init(prop.totalGlobalMem / 64, reinterpret_cast<BufferPool::AddressRange>(range));
     // opt in to large dynamic shared memory once per context (each call is checked by its own return value: a kernel
     // whose static shared memory pushes the sum over the limit must fail here, not at its first launch)
     struct { const void* fn; int bytes; const char* name; } opt_in[] = {
@@ -481,6 +496,13 @@ extern "C" int32_t fusor_cuda_buffer_free(fusor_cuda_ctx* ctx, void* device_ptr)
     CUDA_TRY(ctx, cudaFree(device_ptr));
     return FUSOR_CUDA_OK;
 }
+extern "C" int32_t fusor_cuda_buffer_trim(fusor_cuda_ctx* ctx) {
+    if (!ctx) return fail(nullptr, FUSOR_CUDA_INVALID_ARGUMENT, "ctx is null");
+    DeviceGuard g(ctx->device);
+    if (capturing(ctx)) CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));  // refused, as cudaFree is
+    ctx->pool.drain();
+    return FUSOR_CUDA_OK;
+}
 extern "C" int32_t fusor_cuda_buffer_upload(fusor_cuda_ctx* ctx, void* dst, const void* src, size_t bytes) {
     if (!ctx || (bytes && (!dst || !src))) return fail(ctx, FUSOR_CUDA_INVALID_ARGUMENT, "null argument");
     DeviceGuard g(ctx->device);
@@ -572,6 +594,11 @@ static int32_t validate_attention(fusor_cuda_ctx* ctx, const fusor_cuda_tensor4*
         return fail(ctx, FUSOR_CUDA_SHAPE_MISMATCH, "causal attention needs kv_len (%d) >= q_len (%d)", S->Skv, S->Sq);
     if (mask_kind == FUSOR_CUDA_MASK_SLIDING && window <= 0) return fail(ctx, FUSOR_CUDA_INVALID_ARGUMENT, "window must be positive");
     return FUSOR_CUDA_OK;
+}
+
+// the limit of every call that the tcgen05 kernels do not take
+static int32_t check_heads(fusor_cuda_ctx* ctx, const AttnShape& S) {
+    return S.Hq > 65535 || S.B > 65535 ? fail(ctx, FUSOR_CUDA_UNSUPPORTED, "more than 65535 heads or batches") : FUSOR_CUDA_OK;
 }
 
 // =============================================================================== attention: launches
@@ -721,16 +748,18 @@ static int32_t launch_mma(fusor_cuda_ctx* ctx, const AttnShape& S, const fusor_c
 
 // The softmax weights are kept in f16 against an f16 copy of V (the kernels fall back to bf16 weights and the bf16 V on
 // the device when some |v| does not fit f16).
+// `call_heads`: (batch, query head) pairs that the choice of the kernel counts, those of the whole call where this is a part of
+// it: the bits of a head's result then do not depend on how a call was cut up.
 static int32_t launch_prefill(fusor_cuda_ctx* ctx, const AttnShape& S, const fusor_cuda_tensor4* q,
                               const fusor_cuda_tensor4* k, const fusor_cuda_tensor4* v, float scale, int32_t mask_kind,
-                              const fusor_cuda_tensor4* out, int window = 0, const fusor_cuda_tensor2* key_mask = nullptr,
-                              const fusor_cuda_tensor2* qk_mask = nullptr) {
+                              const fusor_cuda_tensor4* out, int window, const fusor_cuda_tensor2* key_mask,
+                              const fusor_cuda_tensor2* qk_mask, long long call_heads) {
     // Two query tiles per CTA with 128-key blocks once the 256-row items outnumber the SMs; below that its CTAs each have one
     // item and the call lasts as long as the longest, which 128-row tiles on twice the CTAs finish sooner (H32/8 causal, us,
     // two tiles / one: S512 15.9 / 12.7, S1000 24.1 / 20.9, S1500 33.0 / 34.4 with 192 items; H8/8 S4096 67 / 60; B4 S300
     // 21.3 / 18.1, where every second item is half empty).  Calls with an additive [Sq, Skv] mask tensor always take the 64-key
     // kernel (each softmax thread reads a row of mask values per tile: it has the registers for that).
-    const long long items = (long long)((S.Sq + P2_ROWS - 1) / P2_ROWS) * S.Hq * S.B;
+    const long long items = (long long)((S.Sq + P2_ROWS - 1) / P2_ROWS) * call_heads;
     const bool two_tiles = S.Sq > P2_ROWS + P2_BM && items > ctx->num_sms && qk_mask == nullptr;
     const int kv_rows = two_tiles ? P2_BN : PF_BN;
     const bool in_f16 = q->dtype == FUSOR_CUDA_F16;  // f16 tensors need no copy of V: the weights are f16 against V itself
@@ -791,9 +820,9 @@ static int32_t launch_prefill(fusor_cuda_ctx* ctx, const AttnShape& S, const fus
     }
     // Few tiles: parts of the keys on up to 8 CTAs each, two CTAs per SM.  The merge costs as much as four to six key tiles, so
     // the longest row of tiles has to be 16 for two parts, and a part keeps more than 4.5.
-    const long long longest = (std::min(S.Skv, P.window > 0 ? P.window + PF_BM : S.Skv) + PF_BN - 1) / PF_BN;
+    const long long longest = (std::min(S.Skv, P.window > 0 && P.window < S.Skv ? P.window + PF_BM : S.Skv) + PF_BN - 1) / PF_BN;
     int parts = 1;
-    while (parts < PF_MAX_SPLIT && grid * parts * 2 <= 2ll * ctx->num_sms && longest > (parts == 1 ? 15 : 9ll * parts)) parts *= 2;
+    while (parts < PF_MAX_SPLIT && P.n_q_tiles * call_heads * parts * 2 <= 2ll * ctx->num_sms && longest > (parts == 1 ? 15 : 9ll * parts)) parts *= 2;
     if (parts > 1) {
         cudaLaunchAttribute attr;
         const cudaLaunchConfig_t cfg = cluster_config(ctx, (unsigned)(grid * parts), (unsigned)parts, PF_THREADS, PF_SMEM_BYTES, &attr);
@@ -805,18 +834,25 @@ static int32_t launch_prefill(fusor_cuda_ctx* ctx, const AttnShape& S, const fus
     return launch_check(ctx, "prefill_sm100_kernel");
 }
 
-extern "C" int32_t fusor_cuda_flash_attention(fusor_cuda_ctx* ctx, const fusor_cuda_tensor4* q, const fusor_cuda_tensor4* k,
-                                              const fusor_cuda_tensor4* v, float scale, const fusor_cuda_tensor2* mask,
-                                              int32_t mask_kind, int32_t window, const fusor_cuda_tensor4* out) {
+// A call, or (call_heads > 0) a part of one with that many (batch, query head) pairs.
+static int32_t flash_attention(fusor_cuda_ctx* ctx, const fusor_cuda_tensor4* q, const fusor_cuda_tensor4* k, const fusor_cuda_tensor4* v, float scale,
+                               const fusor_cuda_tensor2* mask, int32_t mask_kind, int32_t window, const fusor_cuda_tensor4* out, long long call_heads) {
     AttnShape S;
     TRY(validate_attention(ctx, q, k, v, mask, mask_kind, window, out, &S));
     DeviceGuard g(ctx->device);
     if (prefill_eligible(S, q, k, v, scale, mask_kind, out, mask))
         return launch_prefill(ctx, S, q, k, v, scale, mask_kind, out, window,
                               mask_kind == FUSOR_CUDA_MASK_BATCH_KEY ? mask : nullptr,
-                              mask_kind == FUSOR_CUDA_MASK_QK ? mask : nullptr);
+                              mask_kind == FUSOR_CUDA_MASK_QK ? mask : nullptr, call_heads > 0 ? call_heads : (long long)S.B * S.Hq);
+    TRY(check_heads(ctx, S));
     if (mma_eligible(S, q, k, v, scale, out)) return launch_mma(ctx, S, q, k, v, scale, mask, mask_kind, window, out);
     return launch_general(ctx, S, q, k, v, scale, mask, mask_kind, window, out);
+}
+
+extern "C" int32_t fusor_cuda_flash_attention(fusor_cuda_ctx* ctx, const fusor_cuda_tensor4* q, const fusor_cuda_tensor4* k,
+                                              const fusor_cuda_tensor4* v, float scale, const fusor_cuda_tensor2* mask,
+                                              int32_t mask_kind, int32_t window, const fusor_cuda_tensor4* out) {
+    return flash_attention(ctx, q, k, v, scale, mask, mask_kind, window, out, 0);
 }
 
 extern "C" int32_t fusor_cuda_flash_attention_general(fusor_cuda_ctx* ctx, const fusor_cuda_tensor4* q,
@@ -826,6 +862,7 @@ extern "C" int32_t fusor_cuda_flash_attention_general(fusor_cuda_ctx* ctx, const
     AttnShape S;
     TRY(validate_attention(ctx, q, k, v, mask, mask_kind, window, out, &S));
     DeviceGuard g(ctx->device);
+    TRY(check_heads(ctx, S));
     return launch_general(ctx, S, q, k, v, scale, mask, mask_kind, window, out);
 }
 
@@ -891,11 +928,12 @@ extern "C" int32_t fusor_cuda_attention_out_proj(fusor_cuda_ctx* ctx, const fuso
         return fail(ctx, FUSOR_CUDA_UNSUPPORTED, "the output projection takes bf16 attention output and bf16 weights and writes f32 or bf16");
     if (D % OP_BK != 0) return fail(ctx, FUSOR_CUDA_UNSUPPORTED, "head_dim must be a multiple of %d", OP_BK);
     if (!tma_view_ok(attn)) return fail(ctx, FUSOR_CUDA_UNSUPPORTED, "attention output view is not 16-byte aligned");
-    if (weight->stride[3] != 1 || weight->stride[2] % 8 != 0 || reinterpret_cast<uintptr_t>(weight->data) % 16)
-        return fail(ctx, FUSOR_CUDA_UNSUPPORTED, "weight rows must be contiguous and 16-byte aligned");
+    if (weight->stride[3] != 1 || weight->stride[2] % 8 != 0 || (N > 1 && weight->stride[2] < 0) || reinterpret_cast<uintptr_t>(weight->data) % 16)
+        return fail(ctx, FUSOR_CUDA_UNSUPPORTED, "weight rows must be contiguous, in ascending order and 16-byte aligned");
     const int al = out->dtype == FUSOR_CUDA_F32 ? 4 : 8;
-    if (out->stride[3] != 1 || out->stride[2] % al != 0 || (B > 1 && out->stride[0] % al != 0) || reinterpret_cast<uintptr_t>(out->data) % 16)
-        return fail(ctx, FUSOR_CUDA_UNSUPPORTED, "out rows must be contiguous and 16-byte aligned");
+    if (out->stride[3] != 1 || out->stride[2] % al != 0 || (S > 1 && out->stride[2] < 0) || (B > 1 && (out->stride[0] % al != 0 || out->stride[0] < 0)) ||
+        reinterpret_cast<uintptr_t>(out->data) % 16)
+        return fail(ctx, FUSOR_CUDA_UNSUPPORTED, "out rows must be contiguous, in ascending order and 16-byte aligned");
     if (bias && reinterpret_cast<uintptr_t>(bias) % 4) return fail(ctx, FUSOR_CUDA_INVALID_ARGUMENT, "bias is misaligned");
     DeviceGuard g(ctx->device);
     fusor_cuda_tensor4 w4 = *weight;
@@ -1010,7 +1048,7 @@ extern "C" int32_t fusor_cuda_flash_attention_host(fusor_cuda_ctx* ctx, const fu
             cudaMemcpyAsync(cv.data, (const uint8_t*)v->data + ko * vs, kv_chunk * vs, cudaMemcpyHostToDevice, ctx->h2d_stream);
             cudaEventRecord(in_done, ctx->h2d_stream);
             cudaStreamWaitEvent(ctx->stream, in_done, 0);
-            rc = fusor_cuda_flash_attention(ctx, &cq, &ck, &cv, scale, nullptr, mask_kind, window, &co);
+            rc = flash_attention(ctx, &cq, &ck, &cv, scale, nullptr, mask_kind, window, &co, (long long)S.B * S.Hq);
             if (rc != FUSOR_CUDA_OK) break;
             cudaEventRecord(k_done, ctx->stream);
             cudaStreamWaitEvent(ctx->d2h_stream, k_done, 0);
@@ -1796,8 +1834,8 @@ extern "C" int32_t fusor_cuda_exchange_create(fusor_cuda_ctx* ctx, int32_t world
     ex->ctx = ctx; ex->world = world; ex->rank = rank; ex->slot_floats = (size_t)slot_floats;
     ex->flags_off = align256(2 * (size_t)world * ex->slot_floats * 4);
     const size_t bytes = ex->flags_off + align256(2 * (size_t)world * 8);
-    if (cudaMalloc(&ex->base, bytes) != cudaSuccess || cudaMemset(ex->base, 0, bytes) != cudaSuccess ||
-        cudaMalloc(&ex->done, 256) != cudaSuccess || cudaMemset(ex->done, 0, 256) != cudaSuccess) {
+    if (ctx->pool.plain(bytes, &ex->base) != cudaSuccess || cudaMemset(ex->base, 0, bytes) != cudaSuccess ||
+        ctx->pool.plain(256, reinterpret_cast<void**>(&ex->done)) != cudaSuccess || cudaMemset(ex->done, 0, 256) != cudaSuccess) {
         cudaError_t e = cudaGetLastError();
         if (ex->base) cudaFree(ex->base);
         if (ex->done) cudaFree(ex->done);
@@ -2031,6 +2069,7 @@ extern "C" int32_t fusor_cuda_comm_init(fusor_cuda_ctx* ctx, const void* id128, 
     std::memcpy(&id, id128, 128);
     ncclConfig_t config = NCCL_CONFIG_INITIALIZER;
     config.blocking = 0;  // every call returns at once; completion is polled against the caller's deadline
+    ctx->pool.drain();    // NCCL allocates for itself
     const ncclResult_t r = api->CommInitRankConfig(&cm->comm, world, id, rank, &config);
     if (r != ncclSuccess && r != ncclInProgress) {
         const int32_t rc = fail(ctx, FUSOR_CUDA_NCCL_ERROR, "ncclCommInitRankConfig: %s", api->GetErrorString(r));

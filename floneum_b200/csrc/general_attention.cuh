@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(GEN_THREADS) general_attention_kernel(const __
         }
         // ---- scale, mask, online softmax, in natural units: only differences are taken to log2, so that finite mask values down
         // to the lowest float stay finite
-        const bool edge = kt + GEN_BN > P.Skv || (causal && kt + GEN_BN - 1 > q0 + offset) || (P.mask_kind == 4 && kt + P.window <= q0 + BM - 1 + offset);
+        const bool edge = kt + GEN_BN > P.Skv || (causal && kt + GEN_BN - 1 > q0 + offset) || (P.mask_kind == 4 && kt <= q0 + BM - 1 + offset - P.window);
         __syncwarp();  // the warp has read the P rows of the last tile
 #pragma unroll
         for (int r = 0; r < RT; ++r) {
@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(GEN_THREADS) general_attention_kernel(const __
                     const long long row = P.mask_kind == 1 ? min(qi, P.Sq - 1) : b;
                     s[j] = __fadd_rn(s[j], __ldg(P.mask + row * P.ms[0] + (long long)min(kj, P.Skv - 1) * P.ms[1]));  // rounded as the composite does
                 }
-                if (edge && (kj >= P.Skv || (causal && kj > qi + offset) || (P.mask_kind == 4 && kj + P.window <= qi + offset))) s[j] = -INFINITY;
+                if (edge && (kj >= P.Skv || (causal && kj > qi + offset) || (P.mask_kind == 4 && kj <= qi + offset - P.window))) s[j] = -INFINITY;
                 mx = fmaxf(mx, s[j]);
             }
 #pragma unroll

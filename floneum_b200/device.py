@@ -60,6 +60,10 @@ class Device:
     def free(self, ptr: int):
         self._L.fusor_cuda_buffer_free(self._h, ptr)
 
+    def trim(self):
+        """Gives the freed buffers that are kept for reuse back to the GPU (they come to at most a 64th of its memory)."""
+        _lib.check(self._L.fusor_cuda_buffer_trim(self._h), self._h)
+
     def close(self):
         if getattr(self, "_h", None):
             self._L.fusor_cuda_ctx_destroy(self._h)

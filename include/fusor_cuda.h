@@ -93,6 +93,10 @@ int64_t fusor_cuda_launch_count(fusor_cuda_ctx* ctx);
 
 int32_t fusor_cuda_buffer_alloc(fusor_cuda_ctx* ctx, size_t bytes, void** device_ptr);
 int32_t fusor_cuda_buffer_free(fusor_cuda_ctx* ctx, void* device_ptr);
+/* Freed buffers are kept for the next allocations of their size: at most a 64th of the GPU's memory per context.  This gives
+ * all of them back to the GPU (for another allocator of the process, say); so does destroying the context, and so does the
+ * library where an allocation of its own would fail otherwise.  Waits for the work of every stream, as cudaFree does. */
+int32_t fusor_cuda_buffer_trim(fusor_cuda_ctx* ctx);
 int32_t fusor_cuda_buffer_upload(fusor_cuda_ctx* ctx, void* device_dst, const void* host_src, size_t bytes);
 int32_t fusor_cuda_buffer_download(fusor_cuda_ctx* ctx, void* host_dst, const void* device_src, size_t bytes);
 /* f32 -> bf16 (round to nearest even) / bf16 -> f32 on the device, n contiguous elements. */

@@ -45,6 +45,7 @@ class Device {
         if (rc != FUSOR_CUDA_OK) throw std::runtime_error(fusor_cuda_last_error(ctx_));
     }
     void synchronize() const { check(fusor_cuda_stream_sync(ctx_)); }
+    void trim() const { check(fusor_cuda_buffer_trim(ctx_)); }  // freed buffers kept for reuse go back to the GPU
     int64_t launch_count() const { return fusor_cuda_launch_count(ctx_); }
 
   private:

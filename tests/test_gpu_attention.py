@@ -492,3 +492,28 @@ def test_prefill_f16_tensors(device, B, Hq, Hkv, Sq, Skv, causal):
         got64 = _run(device, q64, k64, v64, 0.125, mask, dtype=2, out_dtype=2)
         assert_close(got64, h(O.flash_attention(q64, k64, v64, 0.125, mask_kind=O.MASK_CAUSAL)), max_tol=2.0 ** -10 + 2e-5, mean_tol=2e-4,
                      what="f16 through the general kernel")
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,S,window", [(1, 32, 8, 1200, 0), (1, 8, 8, 2048, 0), (2, 16, 8, 1100, 300)])
+def test_host_entry_point_takes_the_kernel_of_the_whole_call(device, B, Hq, Hkv, S, window):
+    """The pieces a host call is cut into have fewer heads than the call: two query tiles per CTA or one, and the number of CTAs
+    that share a tile's keys, still follow the whole call, so that the result has the bits of the one-piece device path."""
+    import ctypes
+    from floneum_b200 import _lib
+    fb = _mods()
+    q, k, v, scale = _bf16_case(S + Hq, B, Hq, Hkv, S, S)
+    hq, hk, hv = (np.ascontiguousarray(O.bf16_bits(a)) for a in (q, k, v))
+    out = np.full(q.shape, np.nan, np.float32)
+
+    def t4(a, dtype):
+        t = _lib.Tensor4()
+        t.data, t.dtype = a.ctypes.data, dtype
+        for i in range(4):
+            t.shape[i], t.stride[i] = a.shape[i], a.strides[i] // a.itemsize
+        return t
+    cq, ck, cv, co = t4(hq, _lib.BF16), t4(hk, _lib.BF16), t4(hv, _lib.BF16), t4(out, _lib.F32)
+    assert hq.nbytes + hk.nbytes + hv.nbytes + out.nbytes > (8 << 20)
+    _lib.check(_lib.load().fusor_cuda_flash_attention_host(device.handle, ctypes.byref(cq), ctypes.byref(ck), ctypes.byref(cv), ctypes.c_float(scale), None,
+                                                           _lib.MASK_SLIDING if window else _lib.MASK_CAUSAL, window, ctypes.byref(co)), device.handle)
+    mask = (fb.MaskCache().get_mask(S, 0, window or None, device), fb.MaskKind.QKMask)
+    assert np.array_equal(out, _run(device, q, k, v, scale, mask, dtype=1))

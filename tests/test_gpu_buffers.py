@@ -88,3 +88,87 @@ def test_buffers_while_another_thread_captures_a_graph(device, mode):
         done.set()
         t.join()
     assert got == [3.0]
+
+
+def _cudart():
+    import glob
+    import os
+    import torch
+    return ctypes.CDLL(sorted(glob.glob(os.path.join(os.path.dirname(torch.__file__), "..", "nvidia", "cuda_runtime", "lib", "libcudart.so*")))[0])
+
+
+def _granted(cudart, p):
+    """Bytes of the allocation that starts at p, as the driver knows it."""
+    base, size = ctypes.c_uint64(), ctypes.c_size_t()
+    cuda = ctypes.CDLL("libcuda.so.1")
+    assert cuda.cuMemGetAddressRange_v2(ctypes.byref(base), ctypes.byref(size), ctypes.c_uint64(p)) == 0 and base.value == p
+    return size.value
+
+
+def test_a_buffer_freed_through_another_context_leaves_no_size_behind(device):
+    """Its address may come back with fewer bytes; a release of that one must not enter the pool under the old size."""
+    import torch
+    import floneum_b200 as fb
+    cudart, other = _cudart(), fb.Device.gpu(0)
+    torch.cuda.synchronize()
+    big = 48 << 20
+    p = device.alloc(big)
+    assert _granted(cudart, p) >= big
+    other.free(p)
+    held, got = [], ctypes.c_void_p()
+    for _ in range(400):  # until the driver hands the address out again
+        assert cudart.cudaMalloc(ctypes.byref(got), ctypes.c_size_t(3 << 20)) == 0
+        held.append(got.value)
+        if got.value == p:
+            break
+    for q in held:
+        if q != p:
+            assert cudart.cudaFree(ctypes.c_void_p(q)) == 0
+    if held[-1] != p:
+        pytest.skip("the driver did not hand the address out again")
+    device.free(p)
+    again = [device.alloc(big) for _ in range(12)]
+    try:
+        assert all(_granted(cudart, q) >= big for q in again)
+    finally:
+        for q in again:
+            device.free(q)
+
+
+def test_the_exchange_buffer_may_use_what_is_kept(device):
+    """On a full GPU the bytes that the pool keeps are given back before an allocation of the library fails."""
+    import gc
+    import torch
+    import floneum_b200 as fb
+    from floneum_b200 import _lib
+    L, ex = _lib.load(), ctypes.c_void_p()
+    gc.collect()
+    torch.cuda.empty_cache()
+    mine = fb.Device.gpu(0)
+    held = [mine.alloc(500 << 20) for _ in range(4)]
+    for p in held:
+        mine.free(p)
+    rest = torch.empty(torch.cuda.mem_get_info()[0] - (400 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        assert torch.cuda.mem_get_info()[0] < 900 << 20
+        _lib.check(L.fusor_cuda_exchange_create(mine.handle, 1, 0, 1 << 27, ctypes.byref(ex)), mine.handle)  # two parities of 512 MB
+        L.fusor_cuda_exchange_destroy(ex)
+    finally:
+        del rest
+        torch.cuda.empty_cache()
+
+
+def test_kept_buffers_can_be_asked_back(device):
+    import torch
+    import floneum_b200 as fb
+    mine = fb.Device.gpu(0)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    held = [mine.alloc(500 << 20) for _ in range(4)]
+    for p in held:
+        mine.free(p)
+    assert torch.cuda.mem_get_info()[0] < before - (1 << 30)  # kept
+    mine.trim()
+    assert torch.cuda.mem_get_info()[0] > before - (64 << 20)
+    q = mine.alloc(500 << 20)
+    mine.free(q)
