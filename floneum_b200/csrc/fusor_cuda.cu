@@ -1595,7 +1595,7 @@ static int32_t kv_evict_check(fusor_cuda_kvcache* c, int32_t b, int32_t keep) {
 
 extern "C" int32_t fusor_cuda_kvcache_truncate_front(fusor_cuda_kvcache* c, int32_t b, int32_t keep) {
     TRY(kv_evict_check(c, b, keep));
-    if (keep >= kv_end(c, b)) return FUSOR_CUDA_OK;
+    if (keep >= c->h_kv_len[b] && c->h_front[b] == 0) return FUSOR_CUDA_OK;  // nothing to evict, nothing left to move
     DeviceGuard g(c->ctx->device);
     TRY(kv_keep_rows(c, b, std::min(keep, c->h_kv_len[b])));
     return kv_sync_tables(c);

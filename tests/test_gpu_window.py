@@ -77,6 +77,26 @@ def test_a_pool_with_no_page_to_spare_takes_what_fits(device):
         assert np.array_equal(got[0], k[0, :, 54:]) and not got[1].any()
 
 
+@pytest.mark.parametrize("keep", [0, 20, 33, 38, 1000])
+def test_truncate_front_moves_what_drop_front_left(device, keep):
+    """After truncate_front the first row of the first page is the oldest row kept, also where the call itself evicts nothing."""
+    fb = _fb()
+    rng = np.random.default_rng(keep)
+    T = lambda a: fb.Tensor.from_slice(device, a.shape, np.ascontiguousarray(a))
+    k = O.bf16_round(rng.standard_normal((1, 2, 40, 64), dtype=np.float32))
+    cache = fb.PagedKvCache(device, 1, 2, 64, 6, 4)
+    cache.append(T(k), T(k))
+    cache.drop_front(0, 33)
+    cache.truncate_front(0, keep)
+    n = min(keep, 33)
+    assert cache.seq_len(0) == n
+    pages = cache.read_pages(0, 6)[0].reshape(6, 2, 16, 64)
+    if n:
+        rows = O.bf16_bits(np.ascontiguousarray(k[0, :, 40 - n:40 - n + min(n, 16)]))
+        assert any(np.array_equal(pages[p][:, :min(n, 16)], rows) for p in range(6))
+        assert np.array_equal(cache.gather(1, n)[0].as_slice(), k[:, :, 40 - n:])
+
+
 @pytest.mark.parametrize("B", [1, 32, 33])
 def test_lengths_reach_the_device_with_and_without_a_launch_that_carries_them(device, B):
     """Appends that map no page bring the lengths in their launch (up to 32 sequences); a drop with no append after it, and the
