@@ -48,6 +48,7 @@ SIGNATURES = {
     "fusor_cuda_last_error": (c_char_p, [c_void_p]),
     "fusor_cuda_stream_sync": (c_int32, [c_void_p]),
     "fusor_cuda_launch_count": (c_int64, [c_void_p]),
+    "fusor_cuda_last_kernel": (c_char_p, [c_void_p]),
     "fusor_cuda_buffer_alloc": (c_int32, [c_void_p, c_size_t, POINTER(c_void_p)]),
     "fusor_cuda_buffer_free": (c_int32, [c_void_p, c_void_p]),
     "fusor_cuda_buffer_trim": (c_int32, [c_void_p]),

@@ -208,6 +208,7 @@ struct fusor_cuda_ctx {
     int num_sms = 0;
     int* d_err = nullptr;  // device error word written by kernels
     long long launches = 0;
+    const char* last_kernel = "";
     std::string last_error;
     BufferPool pool;  // results and other buffers of fusor_cuda_buffer_alloc
     PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
@@ -448,6 +449,8 @@ extern "C" const char* fusor_cuda_last_error(fusor_cuda_ctx* ctx) {
 
 extern "C" int64_t fusor_cuda_launch_count(fusor_cuda_ctx* ctx) { return ctx ? ctx->launches : 0; }
 
+extern "C" const char* fusor_cuda_last_kernel(fusor_cuda_ctx* ctx) { return ctx ? ctx->last_kernel : ""; }
+
 static int32_t check_device_error(fusor_cuda_ctx* ctx) {
     int h = 0;
     CUDA_TRY(ctx, cudaMemcpyAsync(&h, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
@@ -521,6 +524,7 @@ static int32_t launch_check(fusor_cuda_ctx* ctx, const char* what) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(ctx, FUSOR_CUDA_CUDA_ERROR, "%s launch failed: %s", what, cudaGetErrorString(e));
     ctx->launches++;
+    ctx->last_kernel = what;
     return FUSOR_CUDA_OK;
 }
 

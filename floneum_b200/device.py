@@ -50,6 +50,10 @@ class Device:
     def launch_count(self) -> int:
         return int(self._L.fusor_cuda_launch_count(self._h))
 
+    def last_kernel(self) -> str:
+        """Name of the kernel launched last."""
+        return self._L.fusor_cuda_last_kernel(self._h).decode()
+
     def alloc(self, nbytes: int) -> int:
         p = ctypes.c_void_p()
         rc = self._L.fusor_cuda_buffer_alloc(self._h, nbytes, ctypes.byref(p))

@@ -90,6 +90,8 @@ const char* fusor_cuda_last_error(fusor_cuda_ctx* ctx);
 int32_t fusor_cuda_stream_sync(fusor_cuda_ctx* ctx);
 /* Number of kernels this context has launched so far. */
 int64_t fusor_cuda_launch_count(fusor_cuda_ctx* ctx);
+/* Name of the kernel this context has launched last ("" before the first): which of several a call of some size takes. */
+const char* fusor_cuda_last_kernel(fusor_cuda_ctx* ctx);
 
 int32_t fusor_cuda_buffer_alloc(fusor_cuda_ctx* ctx, size_t bytes, void** device_ptr);
 int32_t fusor_cuda_buffer_free(fusor_cuda_ctx* ctx, void* device_ptr);
