@@ -11,9 +11,9 @@
 // One CTA = 64 query rows of one (batch, head), 4 warps x 16 rows; K and V tiles of 64 keys come by cp.async into two
 // buffers, rows padded by 16 bytes so that ldmatrix meets no bank conflict; Q stays in registers.  Three CTAs per SM
 // (head_dim 64) hide each other's barriers and softmax.  Bound by the warp MMA pipe (538 TFLOP/s of bf16 products, measured):
-// B4 H32/8 S2048 D64 causal 201 TFLOP/s in f16 and 158 in bf16, three and four MMAs per useful two, 55-59 % of that pipe.
-// Against the f32-arithmetic kernel that served these tensors: B8 H16 S300 D64 f16 with a key mask 852 -> 31 us, B2 H32/8 S1024
-// D64 bf16 causal 2259 -> 64 us; error against 64 bits 2.1e-7 to 3.7e-7 of the norm (f32 arithmetic: 1.7e-7 to 8.7e-7).
+// B4 H32/8 S2048 D64 causal 192 TFLOP/s in f16, three MMAs per useful two (four in bf16), 54 % of that pipe.
+// Against the f32-arithmetic kernel that served these tensors: B8 H16 S300 D64 f16 with a key mask 852 -> 33 us, B2 H32/8 S1024
+// D64 bf16 causal 2259 -> 64 us; error against 64 bits 0.38 to 0.98 times that of f32 arithmetic with its sums in order.
 #pragma once
 #include "ptx_sm100.cuh"
 

@@ -11,16 +11,18 @@
 // tile's copy runs under the MMAs of this one.  Q is split once into planes of its own.
 // B1 H32/8 S512 D64 causal: 35 us (62 us on the CUDA cores in general_attention_kernel); B2 H32/8 S2048 without a mask:
 // 45 TFLOP/s at head_dim 64 and 44 at 128 (30 and 29), half of what the MMA pipe gives at six products; the staging and the
-// split take most of the rest.  Error against 64 bits 1.9e-7 to 3.1e-7 of the norm (CUDA cores: 2.0e-7 to 8.4e-7).
+// split take most of the rest.  Error against 64 bits 0.39 to 0.86 times that of f32 arithmetic with its sums in order.
 #pragma once
 #include "attn_mma16.cuh"
 
 namespace fusor {
 
 template <int DP>
-constexpr int a3_bn = DP <= 64 ? 64 : 32;  // keys per tile: what fits two CTAs (head_dim 64) or one (128) on an SM
+constexpr int a3_bn = DP <= 64 ? 64 : 32;  // keys per tile
 template <int DP>
-constexpr int a3_stage_pitch = DP * 4 + 16;  // bytes of an f32 row
+// Bytes of an f32 row.  The padding serves no access; without it two CTAs of head_dim 64 fit an SM, which was faster for full rows
+// (B4 H16 S300 with a key mask 63.5 -> 54 us) and slower for few causal ones (B1 H32/8 S512 34.9 -> 38.5: heavy blocks pair up).
+constexpr int a3_stage_pitch = DP * 4 + 16;
 template <int DP>
 constexpr size_t a3_smem_bytes = (size_t)am_pitch<DP> * 3 * (AM_BM + 2 * a3_bn<DP>) + (size_t)a3_stage_pitch<DP> * 2 * a3_bn<DP>;
 

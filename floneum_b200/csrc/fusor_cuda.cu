@@ -1708,12 +1708,13 @@ static int32_t decode_impl(fusor_cuda_ctx* ctx, fusor_cuda_kvcache* c, const fus
     // Short sequences: a cluster per (sequence, kv head), one launch.  C: the largest cluster of which all fit at once.
     // Measured (8 KB pages, ns): the cluster takes 4600 + L max(126, 161 CTAs / 128) for a longest share of L pages, the even
     // deal 13900 + 194 per page of an SM's share: 16 sequences of 256 .. 2048 tokens 25 against 27.5 us, of 512 .. 4096 tokens
-    // 46 against 37.  Below DCL_MAX pages most of a cluster has none: those calls keep the two launches that the test of the
-    // call pattern counts.
+    // 46 against 37.  Sequences below kClusterMinPages stay on the deal, whose two launches the test of the call pattern counts for
+    // them; the cluster would be faster there as well (one sequence of 40 tokens 6.5 against 13.3 us, sixteen 6.2 and 15.4).
+    constexpr int kClusterMinPages = 8;
     long long longest = 0;
     for (int b = 0; b < B; ++b) longest = std::max<long long>(longest, pages_of(kv_end(c, b)));
     const long long heads = (long long)B * c->Hkv, unit = 2ll * DEC_PT * c->D * 2;
-    if (mode != 2 && c->decode_ctas == 0 && heads <= ctx->num_sms && longest >= DCL_MAX) {
+    if (mode != 2 && c->decode_ctas == 0 && heads <= ctx->num_sms && longest >= kClusterMinPages) {
         int i = 0;
         while (i < 3 && heads <= ctx->clusters[i + 1]) ++i;
         const int C = 1 << i;

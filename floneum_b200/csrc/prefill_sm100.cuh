@@ -8,10 +8,9 @@
 //               S_j = Q K_j^T   (SS: both operands in shared memory, K-major, N = PF_BN),
 //               O  += P_j V_j   (TS: P read from TMEM, V from shared memory, MN-major, N = 128),
 //               and the next S into the buffer P_j is read from straight after (the pipe runs in issue order).
-//   warps 2..   softmax: PF_TPR threads per query row read S from TMEM, keep the running max / sum, write P
-//               (16-bit) back over S, rescale O in TMEM only when the row max has grown by more than 2^8
-//               (lazy rescale), and finally write O / l.  With two threads per row the two warps that share a
-//               TMEM lane quadrant swap their partial row maxima through shared memory.
+//   warps 2-5   softmax: a thread per query row reads S from TMEM, keeps the running max / sum, writes P
+//               (16-bit) back over S, rescales O in TMEM only when the row max has grown by more than 2^8
+//               (lazy rescale), and finally writes O / l.
 // TMEM columns: S / P buffers from column 0 (PF_SBUF x PF_BN <= 128), O in [128,256).
 // All waits are bounded (ptx_sm100.cuh); on a timeout the CTA unwinds and frees its TMEM.
 //
@@ -39,14 +38,9 @@ namespace fusor {
 #ifndef PF_SBUF_CFG
 #define PF_SBUF_CFG 2
 #endif
-#ifndef PF_TPR_CFG
-#define PF_TPR_CFG 1
-#endif
 constexpr int PF_BM = 128, PF_BN = PF_BN_CFG, PF_D = 128;
 constexpr int PF_SBUF = PF_SBUF_CFG;           // S buffers in TMEM = K / V ring slots
-constexpr int PF_TPR = PF_TPR_CFG;             // softmax threads per query row
-constexpr int PF_CPT = PF_BN / PF_TPR;         // key columns per softmax thread
-constexpr int PF_THREADS = 64 + 128 * PF_TPR;  // warp 0 TMA, warp 1 MMA, then softmax warps (warp % 4 = TMEM lane quadrant)
+constexpr int PF_THREADS = 64 + 128;           // warp 0 TMA, warp 1 MMA, then softmax warps (warp % 4 = TMEM lane quadrant), a thread per query row
 constexpr int PF_Q_BYTES = PF_BM * PF_D * 2;   // two [128][64] halves
 constexpr int PF_Q_HALF = PF_Q_BYTES / 2;
 constexpr int PF_KV_BYTES = PF_BN * PF_D * 2;  // two [PF_BN][64] halves
@@ -54,7 +48,7 @@ constexpr int PF_KV_HALF = PF_KV_BYTES / 2;
 constexpr uint32_t PF_TMEM_COLS = 256;
 constexpr uint32_t PF_COL_S = 0, PF_COL_O = 128;  // S buffer b at PF_COL_S + PF_BN b
 constexpr float PF_RESCALE_THRESHOLD = 8.0f;      // in log2 units
-static_assert(PF_SBUF * PF_BN <= 128 && PF_CPT % 32 == 0 && (PF_TPR == 1 || PF_TPR == 2), "tile configuration");
+static_assert(PF_SBUF * PF_BN <= 128 && PF_BN % 32 == 0, "tile configuration");
 
 struct PrefillParams {
     void* out;
@@ -144,11 +138,9 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
     uint64_t* s_full = bars + 9;    // [2]
     uint64_t* p_full = bars + 11;   // [2]
     uint64_t* pv_done = bars + 13;
-    uint64_t* xch_bar = bars + 14;  // [4] one per TMEM lane quadrant: the two softmax warps of a quadrant meet here
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    float* xch = reinterpret_cast<float*>(bars + 32);  // [3][2 halves][128 rows]: partial maxima (2 buffers), row sums
-    float2* part_ml = reinterpret_cast<float2*>(xch);  // SPLIT: [part][128 rows] (m, l)
+    float2* part_ml = reinterpret_cast<float2*>(bars + 32);  // SPLIT: [part][128 rows] (m, l)
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool use_f16 = P.in_f16 != 0 || (P.v_f16_overflow != nullptr && *P.v_f16_overflow == 0);
@@ -180,10 +172,9 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
             mbar_init(v_full + i, 1);
             mbar_init(v_empty + i, 1);
             mbar_init(s_full + i, 1);
-            mbar_init(p_full + i, 128 * PF_TPR);
+            mbar_init(p_full + i, 128);
         }
         mbar_init(pv_done, 1);
-        for (int i = 0; i < 4; ++i) mbar_init(xch_bar + i, 64);
         *abort_flag = 0;
         mbar_fence_init();
         tma_prefetch_desc(&tmQ);
@@ -277,9 +268,6 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
         }
     } else {
         // ------------------------------------------------------------------ softmax / correction / epilogue
-        // PF_TPR threads per query row; thread `half` owns key columns [half*PF_CPT, (half+1)*PF_CPT) of each
-        // S tile and output columns [half*128/PF_TPR, ...).
-        const int half = (warp - 2) >> 2;
         const int quad = warp & 3;
         const int row = quad * 32 + lane;                        // 0..127 = TMEM lane = query row of the tile
         const uint32_t lane_base = (uint32_t)(quad * 32) << 16;  // this warp's TMEM lane quadrant
@@ -288,20 +276,19 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
         const int k_first = P.window > 0 ? qi + offset - P.window + 1 : 0;      // first key this row may see
         const float c = P.scale_log2;
         const float thr = MASK ? PF_RESCALE_THRESHOLD / c : PF_RESCALE_THRESHOLD;
-        constexpr int OC = 128 / PF_TPR;  // output columns per thread
-        const uint32_t o_tmem = tmem_base + lane_base + PF_COL_O + half * OC;
+        const uint32_t o_tmem = tmem_base + lane_base + PF_COL_O;
         for (int j = 0; j < n_kv && ok; ++j) {
             const int st = j % PF_SBUF;
             const uint32_t s_tmem = tmem_base + lane_base + PF_COL_S + st * PF_BN;
             ok = mbar_wait(s_full + st, (j / PF_SBUF) & 1, abort_flag, P.err);
             if (!ok) break;
             tc_fence_after();
-            float s[PF_CPT];
+            float s[PF_BN];
 #pragma unroll
-            for (int cc = 0; cc < PF_CPT / 32; ++cc)
-                tmem_ld32(s_tmem + half * PF_CPT + cc * 32, *reinterpret_cast<uint32_t(*)[32]>(&s[cc * 32]));
+            for (int cc = 0; cc < PF_BN / 32; ++cc)
+                tmem_ld32(s_tmem + cc * 32, *reinterpret_cast<uint32_t(*)[32]>(&s[cc * 32]));
             tc_wait_ld();
-            const int k0 = (j_begin + j) * PF_BN + half * PF_CPT;
+            const int k0 = (j_begin + j) * PF_BN;
             if (MASK == 1) {
                 // additive key mask of this batch row: (s + mask / scale) * scale = s * scale + mask; every thread of the
                 // CTA reads the same values (broadcast loads); keys past Skv are cut by the edge mask below
@@ -314,9 +301,9 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
                 const float* mr = P.qkmask + (long long)min(qi, P.Sq - 1) * P.qkmask_stride;
                 prefill_add_mask(P, mr, k0, s);
             }
-            if (k0 + PF_CPT - 1 > k_limit || k0 < k_first) {  // diagonal, ragged or window-edge tile: mask in the raw domain
+            if (k0 + PF_BN - 1 > k_limit || k0 < k_first) {  // diagonal, ragged or window-edge tile: mask in the raw domain
 #pragma unroll
-                for (int i = 0; i < PF_CPT; ++i)
+                for (int i = 0; i < PF_BN; ++i)
                     if (k0 + i > k_limit || k0 + i < k_first) s[i] = -INFINITY;
             }
             float mx[8];
@@ -325,18 +312,10 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
 #pragma unroll
             for (int a = 0; a < 8; ++a) mx[a] = fmax3(mx[a], s[4 * a + 2], s[4 * a + 3]);
 #pragma unroll
-            for (int i = 32; i < PF_CPT; i += 16)
+            for (int i = 32; i < PF_BN; i += 16)
 #pragma unroll
                 for (int a = 0; a < 8; ++a) mx[a] = fmax3(mx[a], s[i + 2 * a], s[i + 2 * a + 1]);
             float pmax = fmaxf(fmax3(mx[0], mx[1], mx[2]), fmaxf(fmax3(mx[3], mx[4], mx[5]), fmaxf(mx[6], mx[7])));
-            if (PF_TPR == 2) {
-                // swap partial maxima with the thread that owns the other columns of this row
-                xch[((j & 1) * 2 + half) * 128 + row] = pmax;
-                mbar_arrive(xch_bar + quad);
-                ok = mbar_wait(xch_bar + quad, j & 1, abort_flag, P.err);
-                if (!ok) break;
-                pmax = fmaxf(pmax, xch[((j & 1) * 2 + (half ^ 1)) * 128 + row]);
-            }
             const float tmax = MASK ? pmax : pmax * c;  // scale > 0
             // lazy rescale: keep the reference max until the true max has moved by more than the threshold
             const float m_new = (tmax > m_ref + thr) ? tmax : m_ref;  // also taken on the first tile
@@ -352,7 +331,7 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
             const float2 c2 = make_float2(c, c), nm2 = make_float2(-m_sub, -m_sub);
             float2 ps0 = make_float2(0.0f, 0.0f), ps1 = make_float2(0.0f, 0.0f);
 #pragma unroll
-            for (int cc = 0; cc < PF_CPT / 32; ++cc) {
+            for (int cc = 0; cc < PF_BN / 32; ++cc) {
                 uint32_t pk[16];
 #pragma unroll
                 for (int i = 0; i < 16; i += 2) {
@@ -365,7 +344,7 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
                     pk[i] = use_f16 ? pack_f16(p0.x, p0.y) : pack_bf16(p0.x, p0.y);
                     pk[i + 1] = use_f16 ? pack_f16(p1.x, p1.y) : pack_bf16(p1.x, p1.y);
                 }
-                tmem_st16(s_tmem + (half * PF_CPT) / 2 + cc * 16, pk);  // P overwrites the first PF_BN/2 columns of this S buffer
+                tmem_st16(s_tmem + cc * 16, pk);  // P overwrites the first PF_BN/2 columns of this S buffer
             }
             l = l * alpha + ((ps0.x + ps0.y) + (ps1.x + ps1.y));
             tc_wait_st();
@@ -377,7 +356,7 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
                 if (__any_sync(0xffffffffu, alpha != 1.0f)) {
                     const float2 a2 = make_float2(alpha, alpha);
 #pragma unroll
-                    for (int cc = 0; cc < OC / 32; ++cc) {
+                    for (int cc = 0; cc < 128 / 32; ++cc) {
                         float orr[32];
                         tmem_ld32(o_tmem + cc * 32, *reinterpret_cast<uint32_t(*)[32]>(&orr[0]));
                         tc_wait_ld();
@@ -395,13 +374,6 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
             tc_fence_before();
             mbar_arrive(p_full + st);
         }
-        // the row sum is the sum over the row's threads (they used the same sequence of reference maxima)
-        if (PF_TPR == 2 && ok) {
-            xch[(2 * 2 + half) * 128 + row] = l;
-            mbar_arrive(xch_bar + quad);
-            ok = mbar_wait(xch_bar + quad, n_kv & 1, abort_flag, P.err);
-            if (ok) l += xch[(2 * 2 + (half ^ 1)) * 128 + row];
-        }
         if (ok && (!SPLIT || n_kv > 0)) ok = mbar_wait(pv_done, (n_kv - 1) & 1, abort_flag, P.err);
         // Epilogue: O / l goes through shared memory (the Q / K / V buffers are idle once the last MMA has
         // completed) in the 128-byte-swizzled layout of the output tensor map, then out with TMA stores:
@@ -411,11 +383,11 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
             tc_fence_after();
             const float inv_l = 1.0f / l;
 #pragma unroll
-            for (int cc = 0; cc < OC / 32; ++cc) {
+            for (int cc = 0; cc < 128 / 32; ++cc) {
                 float orr[32];
                 tmem_ld32(o_tmem + cc * 32, *reinterpret_cast<uint32_t(*)[32]>(&orr[0]));
                 tc_wait_ld();
-                const int col0 = half * OC + cc * 32;  // first output column of this chunk
+                const int col0 = cc * 32;  // first output column of this chunk
                 if (P.out_dtype == 0) {
                     // f32: 32 columns = one 128-byte block row = 8 chunks of 16 bytes
                     uint8_t* blk = base + (col0 / 32) * BLK_BYTES + row * 128;
@@ -439,7 +411,7 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
             fence_proxy_async_smem();
         }
         // every softmax thread reaches this barrier, also after a timeout (then nothing is stored)
-        const int any_failed = named_bar_or(1, 128 * PF_TPR, ok ? 0 : 1);
+        const int any_failed = named_bar_or(1, 128, ok ? 0 : 1);
         ok = !any_failed;
         if (!SPLIT && ok && warp == 2 && lane == 0) {
             const int n_blk = P.out_dtype == 0 ? 4 : 2, blk_cols = P.out_dtype == 0 ? 32 : 64;
@@ -449,7 +421,6 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
     }
     if (SPLIT) {
         // ------------------------------------------------------------------ the parts of the tile meet
-        static_assert(PF_TPR == 1, "a softmax thread owns a row");
         const int quad = warp & 3, row = quad * 32 + lane;
         const uint32_t o_row = tmem_base + ((uint32_t)(quad * 32) << 16) + PF_COL_O;
         __syncwarp();
