@@ -17,7 +17,7 @@ under a deadline (EXTRAS_DEADLINE_S): should one never return, rank 0 still prin
 measurement and the extras that finished, names the one that did not, and every rank leaves with exit code 0; the
 program's NCCL communicators keep in-switch reduction (NVLS) off unless NCCL_NVLS_ENABLE is set by the caller.
 stdout carries the JSON line only; progress and library chatter go to stderr.
-`--workload cfg1` runs the CPU-reference configuration (f32, general kernel) with the CPU port timed in full.
+`--workload cfg1` runs the CPU-reference configuration (f32, warp-MMA kernel) with the CPU port timed in full.
 `--impl reference` times the CPU restatement of the reference's attention (oracle/) on the host cores instead.
 """
 from __future__ import annotations

@@ -110,17 +110,22 @@ int32_t fusor_cuda_cast(fusor_cuda_ctx* ctx, void* dst, int32_t dst_dtype, const
  * (fusor-ml/core/src/composite/flash_attention.rs:28-52,56-557).
  *   q [B,Hq,Sq,D], k and v [B,Hkv,Skv,D], out [B,Hq,Sq,D]; Hq % Hkv == 0, query head h reads kv head h/(Hq/Hkv).
  *   out = softmax(q k^T * scale + mask) v, f32 accumulation.
- * Dispatch: q/k/v all bf16 or all f16 with D == 128 run the tcgen05 tensor-core kernels: two query tiles per CTA from
- * Sq = 256 and one below for an analytic mask (NONE / CAUSAL / SLIDING) or a [B, Skv] key mask (MASK_BATCH_KEY, rows
- * contiguous); the one-tile kernel at any Sq for an additive [Sq, Skv] mask tensor (MASK_QK, rows contiguous; every key
- * tile is visited and each row reads its mask values).  Everything else (f32 inputs, mixed types, any other D <= 256,
- * strided mask rows) runs the general kernel in f32 arithmetic.  out dtype f32, bf16 or f16.  `mask` is read only for MASK_QK / MASK_BATCH_KEY;
- * `window` only for MASK_SLIDING. */
+ * Dispatch: q/k/v all bf16 or all f16 with D == 128, rows 16-byte aligned and scale > 0 run the tcgen05 tensor-core kernels:
+ * two query tiles per CTA where the call has Sq > 384 and more 256-row items (over heads and batches) than the GPU has SMs,
+ * one below that, its keys shared by a cluster of CTAs where there are few tiles; an additive [Sq, Skv] mask tensor (MASK_QK,
+ * rows contiguous) always runs the one-tile kernel (every key tile is visited and each row reads its mask values).  f32
+ * tensors, and 16-bit tensors those kernels do not take, of one type, D <= 128 a multiple of 8, aligned rows and scale > 0 run
+ * on warp-level MMAs with the accuracy of f32 arithmetic; everything else (mixed types, any other D <= 256, unaligned views)
+ * in f32 arithmetic on the CUDA cores; these two refuse more than 65535 heads or batches.  out dtype f32, bf16 or f16.
+ * The last bits of a head's result can depend on how many heads and batches the call has, since the kernel does.
+ * Mask values may be -inf (a key with no weight; a row of nothing else is NaN) or finite down to the lowest float (a row of
+ * nothing else is the mean of V).  `mask` is read only for MASK_QK / MASK_BATCH_KEY; `window` only for MASK_SLIDING. */
 int32_t fusor_cuda_flash_attention(fusor_cuda_ctx* ctx, const fusor_cuda_tensor4* q, const fusor_cuda_tensor4* k,
                                    const fusor_cuda_tensor4* v, float scale, const fusor_cuda_tensor2* mask,
                                    int32_t mask_kind, int32_t window, const fusor_cuda_tensor4* out);
 
-/* The same call for tensors in HOST memory: uploads q, k, v (and the mask), runs, downloads `out`, synchronises.
+/* The same call for tensors in HOST memory: uploads q, k, v (and the mask), runs, downloads `out`, synchronises.  The result has
+ * the bits of the call on device memory.
  * This is the path of a caller that holds CPU tensors, as the reference's as_slice().await round trip
  * (fusor-ml/fusor/src/lib.rs:391-403). */
 int32_t fusor_cuda_flash_attention_host(fusor_cuda_ctx* ctx, const fusor_cuda_tensor4* q, const fusor_cuda_tensor4* k,
@@ -138,8 +143,8 @@ int32_t fusor_cuda_flash_attention_general(fusor_cuda_ctx* ctx, const fusor_cuda
  * whole GPU to its own memory pool at start-up, where a cudaMalloc from inside this library would fail, or a
  * latency-critical loop that cannot afford the device-wide synchronisation cudaMalloc and cudaFree imply.
  * fusor_cuda_flash_attention grows a context-owned f16 copy of V with cudaMalloc when a larger V arrives; this
- * variant runs the V pre-pass and the 64-key tensor-core prefill kernel (whatever Sq is; the allocating entry point
- * switches to the two-tile kernel from Sq = 256, so the two agree within the tolerance of the path, not bit for bit)
+ * variant runs the V pre-pass and the 64-key tensor-core prefill kernel without shared keys (whatever Sq is; the allocating
+ * entry point chooses by the number of tiles, so the two agree within the tolerance of the path, not always bit for bit)
  * with that copy in a fixed array inside the library image (8 MiB + 256 bytes per GPU, held by every GPU that loads
  * the library until the process exits).
  *   - Needs no context: it runs on the CURRENT device, on `stream` (NULL = the default stream).
@@ -209,7 +214,7 @@ int32_t fusor_cuda_kvcache_truncate_front(fusor_cuda_kvcache* cache, int32_t b, 
 /* The same eviction without moving rows: whole pages go back to the pool, and a remainder of up to 15 evicted rows stays
  * at the front of the sequence's first page, where every operation on the cache skips it (the raw pools show it).  The
  * rows move only when an append would otherwise need a page that the sequence or the pool does not have, or at the next
- * fusor_cuda_kvcache_truncate_front. */
+ * fusor_cuda_kvcache_truncate_front, whatever its `keep`. */
 int32_t fusor_cuda_kvcache_drop_front(fusor_cuda_kvcache* cache, int32_t b, int32_t keep);
 /* KvCache::current_seq_len (kv_cache.rs:65-67) of sequence b. */
 int32_t fusor_cuda_kvcache_seq_len(fusor_cuda_kvcache* cache, int32_t b, int32_t* len);
@@ -235,7 +240,8 @@ int32_t fusor_cuda_kvcache_gather(fusor_cuda_kvcache* cache, const fusor_cuda_te
  * models/kalosm-llama/src/raw/attention_layer.rs:405-448; all-zero mask [1, kv_len]).
  *   q [B,Hq,1,D] (bf16, f16 or f32; rounded to bf16, the type of the cached keys), out [B,Hq,1,D] (f32, bf16 or f16;
  *   rows start on a multiple of four elements).
- * Split-KV: the pages of all (sequence, kv head) pairs are dealt evenly to a persistent grid by the kernel itself, from
+ * Up to as many (sequence, kv head) pairs as SMs, with a longest sequence from 8 pages to a few thousand tokens: one launch, a
+ * cluster of CTAs per pair.  Else split-KV: the pages of all (sequence, kv head) pairs are dealt evenly to a persistent grid by the kernel itself, from
  * the lengths on the device (a step after an append plans and uploads nothing on the host); each CTA emits a partial
  * (m, l, O) per run of pages, and a second kernel, which finds each head's partials with the same deal, merges them by
  * log-sum-exp. */
@@ -288,7 +294,8 @@ int32_t fusor_cuda_exchange_lse_combine(fusor_cuda_exchange* ex, const float* re
  * (models/kalosm-llama/src/raw/attention_layer.rs:450-454, fusor-ml/fusor/src/layers/linear.rs:72-115; the reference
  * multiplies by a GGUF-quantised QMatrix, here the weight is dense).  attn [B,Hq,S,D] bf16 as flash_attention wrote it
  * (no transposed copy is made), weight bf16 given as a tensor4 of shape [1, 1, N, Hq*D] (rows contiguous), bias f32 [N] on the device or NULL, out f32 or bf16 given
- * as a tensor4 of shape [B, 1, S, N].  Products accumulate in f32 on the tensor cores.  With the query heads split over
+ * as a tensor4 of shape [B, 1, S, N].  Products accumulate in f32 on the tensor cores; few rows or tiles split K over CTAs, so
+ * the order of a sum depends on the call's size.  With the query heads split over
  * GPUs each rank passes its heads and the matching columns of the weight and gets a partial sum (bias on one rank only);
  * the ranks then add their results (all-reduce). */
 int32_t fusor_cuda_attention_out_proj(fusor_cuda_ctx* ctx, const fusor_cuda_tensor4* attn, const fusor_cuda_tensor4* weight,

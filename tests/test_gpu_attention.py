@@ -393,8 +393,8 @@ def test_host_entry_point_pipelined_chunks_match_device_path(device):
 @pytest.mark.parametrize("B,Hq,Hkv,S,neg", [(3, 4, 2, 200, -np.inf), (2, 8, 8, 512, -10000.0), (4, 4, 1, 333, -np.inf)])
 def test_batch_key_mask_on_the_tensor_core_kernels(device, B, Hq, Hkv, S, neg):
     """MaskKind::BatchKeyMask ([B, Skv] additive padding mask, bidirectional attention; rbert's Qwen embedding uses -10000,
-    models/rbert/src/raw/qwen/attention.rs:93-113) through the tcgen05 kernels (64-key kernel below 256 rows, two-tile
-    kernel from 256), against the composite with the same mask."""
+    models/rbert/src/raw/qwen/attention.rs:93-113) through the one-tile tcgen05 kernel (too few items for the two-tile one, whose
+    masks test_gpu_attention_two_tile.py covers), against the composite with the same mask."""
     fb = _mods()
     q, k, v, scale = _bf16_case(900 + S, B, Hq, Hkv, S, S)
     rng = np.random.default_rng(S)
@@ -413,7 +413,7 @@ def test_batch_key_mask_on_the_tensor_core_kernels(device, B, Hq, Hkv, S, neg):
 
 @pytest.mark.parametrize("it", range(10))
 def test_prefill_two_tile_kernel_shape_fuzz(device, it):
-    """Seeded shapes for the two-tile kernel (Sq >= 256): ragged query and key counts, key offsets (Skv > Sq), no mask /
+    """Seeded shapes for the tcgen05 kernels (few items: the one-tile kernel; see test_gpu_attention_two_tile.py for the other): ragged query and key counts, key offsets (Skv > Sq), no mask /
     causal / sliding window / key mask, GQA groups 1-4, against the composite."""
     fb = _mods()
     rng = np.random.default_rng(7000 + it)

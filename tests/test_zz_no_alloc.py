@@ -42,10 +42,8 @@ def test_noalloc_matches_the_allocating_entry_point_twice(device):
     from oracle import oracle as O
     rng = np.random.default_rng(424242)
     scale = float(1.0 / np.sqrt(128.0))
-    # two calls in a row with different shapes and values: the second one meets the first one's leftovers.  The first
-    # shape sends the allocating entry point to the two-tile kernel (Sq >= 256) while this one always runs the 64-key
-    # kernel, so the two agree within the tolerance of the path; the second shape runs the same kernel in both and
-    # must agree bit for bit.
+    # two calls in a row with different shapes and values: the second one meets the first one's leftovers.  Calls of
+    # so few tiles run the one-tile kernel, unsplit, in the allocating entry point too.
     for (B, Hq, Hkv, Sq, Skv, kind) in [(2, 8, 2, 300, 300, _lib.MASK_CAUSAL), (1, 4, 4, 130, 517, _lib.MASK_NONE)]:
         q = W.bf16_round(rng.standard_normal((B, Hq, Sq, 128), dtype=np.float32))
         k = W.bf16_round(rng.standard_normal((B, Hkv, Skv, 128), dtype=np.float32))
