@@ -180,16 +180,7 @@ __global__ void __launch_bounds__(AM_THREADS, DP <= 64 ? 2 : 1) attn_mma32_kerne
             }
         }
         // ---- additive masks (natural units), then the tile's edges (causal diagonal, window, past the last key)
-        if (ADD) {
-#pragma unroll
-            for (int nt = 0; nt < BN / 8; ++nt) {
-                const int kj = kt + nt * 8 + cq;
-                const float* k0 = mask0 + (long long)min(kj, P.Skv - 1) * P.ms[1];
-                const float* k1 = mask0 + (long long)min(kj + 1, P.Skv - 1) * P.ms[1];
-                am_add_mask(s[nt][0], s[nt][1], P.scale, __ldg(k0), __ldg(k1));
-                am_add_mask(s[nt][2], s[nt][3], P.scale, __ldg(k0 + mask_row8), __ldg(k1 + mask_row8));
-            }
-        }
+        if (ADD) am_add_mask_tile<BN>(P, mask0, mask_row8, kt, cq, s);
         if (kt + BN > P.Skv || (causal && kt + BN - 1 > q0 + warp * 16 + offset) ||
             (P.mask_kind == 4 && kt <= q0 + warp * 16 + 15 + offset - P.window)) {
 #pragma unroll

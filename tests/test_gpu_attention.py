@@ -3,7 +3,7 @@
 They follow the reference's own attention tests (fusor-ml/core/src/composite/flash_attention.rs:559-1060,
 fusor-ml/fusor/src/composite/flash_attention.rs:203-360) with seeded data and the oracle as the expected value.
 Tolerance of the path: max-abs <= 2e-3 and mean-abs <= 2e-4 against the f32 oracle on the same
-(bf16-rounded where the kernel takes bf16) inputs; f32 inputs through the general kernel are held to 2e-5."""
+(bf16-rounded where the kernel takes bf16) inputs; f32 inputs (kernels of f32 accuracy) are held to 2e-5."""
 import numpy as np
 import pytest
 
